@@ -77,6 +77,9 @@ struct s2l_tail_model {
     double real_bytes = 8.0;
     double smem_cap = (double)S2L_SWEEP_SMEM_CAP;
     int chain = S2L_CHAIN_DEFAULT;  // chain block rows (1 = no blocking)
+    bool fold = true;        // the blocks' inverses are folded into their rows (dataflow sweeps)
+    double index_bytes = 4.0;
+    double slot_bytes = 9.0;  // shared memory of a sweep per sparse row
 };
 const char* kProfNames[PC_N] = {"spmv", "local_solve", "coarse", "combine", "krylov_vec"};
 
@@ -182,6 +185,22 @@ struct s2l_setup {
     void* d_binv[2] = {nullptr, nullptr};
     int32_t* d_col[2] = {nullptr, nullptr};
     int32_t* d_u2l = nullptr;
+    // Level sweeps (nlay > 0; else the dataflow sweeps above): layout 0 for one column, layout 1, when
+    // nlay is 2, for blocks of columns
+    struct LevelLay {
+        int cs = 1, slots = 0, kc_max = 1;  // CTAs per subdomain, slots of x and s, right-hand sides per CTA
+        unsigned char* ent[2] = {nullptr, nullptr};
+        uint4* task[2] = {nullptr, nullptr};
+        LevelWarp* warp[2] = {nullptr, nullptr};
+        void* dinv[2] = {nullptr, nullptr};
+        uint16_t *rslot[2] = {nullptr, nullptr}, *bout[2] = {nullptr, nullptr}, *pos = nullptr;
+        int32_t *gin = nullptr, *pin = nullptr, *u2l = nullptr, *gout = nullptr;  // as those of the dataflow sweeps
+        // refactorization: sources of the values and of 1/diag, per block its rows, W and the places of W^-1
+        int32_t *src[2] = {nullptr, nullptr}, *dsrc[2] = {nullptr, nullptr}, *bk[2] = {nullptr, nullptr};
+        int64_t *boff[2] = {nullptr, nullptr}, *wsrc[2] = {nullptr, nullptr}, *wpos[2] = {nullptr, nullptr};
+        int64_t nblk[2] = {0, 0};
+    } lay[2];
+    int nlay = 0;
     void* d_val[2] = {nullptr, nullptr};
     void* d_dinv[2] = {nullptr, nullptr};
     int32_t *d_tr_sub = nullptr, *d_tr_i = nullptr, *d_lts_col = nullptr;
@@ -197,7 +216,8 @@ struct s2l_setup {
     // options (s2l_gpu_setup_option)
     int opt_tail_min = 64, opt_tail_max = 4096, opt_group = 0, opt_tail_rows = 0, opt_chain = S2L_CHAIN_DEFAULT, opt_block_width = 0,
         opt_tpr = 0, opt_epl = 4;
-    double opt_hop_us = 0.25, opt_bw_gbs = 6000.0;
+    int opt_level = -1;  // level sweeps: -1 where they are faster, 0 never, 1 wherever they fit
+    double opt_hop_us = 0.0, opt_bw_gbs = 6000.0;  // hop_us 0: the sweeps' default
     std::atomic<int> opt_spin_limit{S2L_SPIN_LIMIT};  // polls of a sweep wait before it gives up
     std::atomic<int> opt_spin_sleep{S2L_SPIN_SLEEP_NS};  // back-off of a sweep poll that found a column not ready
     std::atomic<int> opt_sweep_pf{S2L_BATCH_CHUNKS};     // chunks a sweep warp hints into L2 ahead of its task
@@ -809,11 +829,13 @@ void build_sweep(const HostCsr& M, int T, bool lower, bool unit_diag, int nw, in
     }
 }
 
+#include "level_layout.inl"
+
 // Tail split of one subdomain: T minimising  2 hop levels(T) + bytes(T) nsub / bw, where levels is
 // the dependency depth of the sparse rows < T (forward levels of L, a row's level depends on
 // smaller rows only) and bytes what one local solve reads for this split: sparse entries of L and
 // U, coupling entries L(T:n, 0:T) and U(0:T, T:n), and the two dense triangles of the tail.  The
-// tail is at most tail_max rows; the sweep's shared memory must hold T rows.
+// tail is at most tail_max rows; the sweep's shared memory must hold T rows.  *levels: those of T.
 // Lanes of the U-coupling kernel for a row of `len` entries: about four entries per lane, a power
 // of two, 1 to 32 (a warp takes 32 / lanes rows of about that length)
 int coupling_lanes(int len)
@@ -823,9 +845,8 @@ int coupling_lanes(int len)
     return g;
 }
 
-int choose_tail(const HostCsr& L, const HostCsr& U, int n, const s2l_tail_model& tm)
+int choose_tail(const HostCsr& L, const HostCsr& U, int n, const s2l_tail_model& tm, int* levels)
 {
-    if (tm.force_rows > 0) return std::max(1, n - std::min(tm.force_rows, n - 1));
     // forward levels of L after chain blocking, and the entries blocking adds to each row
     std::vector<int32_t> level(n, 0), extra(n, 0);
     {
@@ -849,12 +870,17 @@ int choose_tail(const HostCsr& L, const HostCsr& U, int n, const s2l_tail_model&
                     }
                 }
                 level[r] = lv;
-                if (B.size() > 1) extra[r] = uni - raw;
+                if (B.size() > 1 && tm.fold) extra[r] = uni - raw;
             }
         }
     }
     std::vector<int32_t> maxlev(n + 1, 0);  // levels of rows [0, T)
     for (int r = 0; r < n; ++r) maxlev[r + 1] = std::max(maxlev[r], level[r] + 1);
+    if (tm.force_rows > 0) {
+        const int T = std::max(1, n - std::min(tm.force_rows, n - 1));
+        *levels = maxlev[T];
+        return T;
+    }
     // entry counts as functions of T (difference arrays)
     std::vector<double> sp(n + 2, 0.0), cp(n + 2, 0.0);
     auto account = [&](const HostCsr& M, bool lower) {
@@ -873,7 +899,7 @@ int choose_tail(const HostCsr& L, const HostCsr& U, int n, const s2l_tail_model&
     account(L, true);
     account(U, false);
     for (int r = 0; r < n; ++r) sp[r + 1] += 2.0 * extra[r];  // fill of the blocked rows (L and U alike)
-    const double rs = tm.real_bytes, idx = 4.0;
+    const double rs = tm.real_bytes, idx = 4.0;  // index bytes of the coupling entries
     double best = 1e300;
     int bestT = n;
     double spc = 0.0, cpc = 0.0;
@@ -887,14 +913,15 @@ int choose_tail(const HostCsr& L, const HostCsr& U, int n, const s2l_tail_model&
     for (int T = n; T >= std::max(1, n - tm.tail_max); --T) {
         const double sz = n - T;
         if (sz > 0 && sz < tm.tail_min) continue;
-        if ((double)T * (rs + 1.0) + 64.0 > tm.smem_cap) continue;
-        const double bytes = (spT[T] + cpT[T]) * (rs + idx) + sz * (sz + 1.0) * rs + 2.0 * T * (rs + 2.0);
+        if ((double)T * tm.slot_bytes + 64.0 > tm.smem_cap) continue;
+        const double bytes = spT[T] * (rs + tm.index_bytes) + cpT[T] * (rs + idx) + sz * (sz + 1.0) * rs + 2.0 * T * (rs + 2.0);
         const double cost = 2.0 * tm.hop_s * maxlev[T] + bytes * tm.nsub / tm.bw;
         if (cost < best) {
             best = cost;
             bestT = T;
         }
     }
+    *levels = maxlev[bestT];
     return bestT;
 }
 
@@ -1027,6 +1054,211 @@ int upload_real(s2l_setup* s, void** dst, const std::vector<double>& v)
 }
 
 // ------------------------------------------------------------------------------ profiling
+// The layouts of the level sweeps, built and uploaded; mpos(i, f): factor positions of the entries of
+// factor f of subdomain i (refactorization) or nullptr, fsize(i): entries of its factor pattern.
+// S2L_ERR_STATE: x and s do not fit the shared memory (or 16-bit slots).
+int build_level_layouts(s2l_setup* s, const std::vector<HostCsr>& Us, const std::vector<int>& Ts,
+                        const std::function<const std::vector<int32_t>*(int, int)>& mpos,
+                        const std::function<int64_t(int)>& fsize, int cap)
+{
+    const int nsub = s->nsub, warps = S2L_BS_LEVEL / 32, gmax = s->opt_group ? s->opt_group : 32;
+    const bool track = mpos(0, 0) != nullptr;
+    const size_t rs = s->real == S2L_REAL_F32 ? 4 : 8, sb = (size_t)level_step_bytes(rs);
+    std::vector<int64_t> loc(nsub + 1, 0), fb(nsub + 1, 0);
+    int max_T = 0;
+    for (int i = 0; i < nsub; ++i) {
+        loc[i + 1] = loc[i] + s->hs[i].n_local();
+        fb[i + 1] = fb[i] + (track ? fsize(i) : 0);
+        max_T = std::max(max_T, Ts[i]);
+    }
+    if (level_smem_bytes(rs, max_T + 1, 1, 2) > S2L_SWEEP_SMEM_CAP) return S2L_ERR_STATE;
+    // CTAs per subdomain: the most, up to S2L_LEVEL_CS, with `groups` clusters of every subdomain on the
+    // device at once.  A stage costs two barriers' time however little it holds, so more CTAs pay while
+    // they run together and cost when they do not: bubbles3d 100^3 / 64, FP32, one column (64 clusters)
+    // 813 us a local solve with 2 CTAs, 886 with 1; four columns (128 clusters) 1539 and 1374.
+    auto ctas = [&](int groups, int most) {
+        for (int c = most; c > 1; c /= 2)
+            if (level_sweep_clusters(rs, max_T + 1, c) >= nsub * groups) return c;
+        return 1;
+    };
+    int kc = 1;
+    while (kc < 4 && level_smem_bytes(rs, max_T + 1, 2 * kc, 2) <= S2L_SWEEP_SMEM_CAP) kc *= 2;
+    // Blocks are sized for four columns, on at most four CTAs (a result goes to every CTA of the cluster:
+    // poisson2d 200^2 / 8, FP64, four columns: 149 us with 4 CTAs, 229 with 8).
+    const int cs[2] = {ctas(1, S2L_LEVEL_CS), ctas(4 / kc, S2L_LEVEL_CS / 2)};
+    const int nlay = cs[1] == cs[0] ? 1 : 2;
+    double bytes = 0.0;
+    auto build = [&](int v) -> int {
+        auto& y = s->lay[v];
+        y.cs = cs[v];
+        const int nw = y.cs * warps;
+        std::vector<LevelSweep> lev[2] = {std::vector<LevelSweep>(nsub), std::vector<LevelSweep>(nsub)};
+        std::vector<std::string> err(nsub);
+        parallel_for(nsub, [&](int i) {
+            const HostSub& h = s->hs[i];
+            build_level_sweep(h.L, Ts[i], true, h.kind != S2L_FACTOR_LLT, y.cs, warps, gmax, s->opt_epl, cap, h.pin,
+                              lev[0][i], err[i], mpos(i, 0));
+            std::vector<int32_t> rows(Ts[i]);  // the backward sweep reads ybuf by rows
+            for (int r = 0; r < Ts[i]; ++r) rows[r] = r;
+            if (err[i].empty())
+                build_level_sweep(Us[i], Ts[i], false, false, y.cs, warps, gmax, s->opt_epl, cap, rows, lev[1][i], err[i],
+                                  mpos(i, 1));
+        });
+        y.slots = 0;
+        for (int i = 0; i < nsub; ++i) {
+            if (err[i].rfind("level sweep:", 0) == 0) return S2L_ERR_STATE;
+            if (!err[i].empty()) return s->fail(S2L_ERR_NUMERIC, "subdomain " + std::to_string(i) + ": " + err[i]);
+            for (int f = 0; f < 2; ++f) y.slots = std::max(y.slots, Ts[i] + 1 + lev[f][i].smax);
+        }
+        if (level_smem_bytes(rs, y.slots, 1, 2) > S2L_SWEEP_SMEM_CAP) {
+            return S2L_ERR_STATE;
+        }
+        y.kc_max = 1;
+        while (y.kc_max < 4 && level_smem_bytes(rs, y.slots, 2 * y.kc_max, 2) <= S2L_SWEEP_SMEM_CAP) y.kc_max *= 2;
+        std::vector<int32_t> gin((size_t)loc[nsub]), pin((size_t)loc[nsub]), u2l((size_t)loc[nsub], 0), gout((size_t)loc[nsub]);
+        std::vector<uint16_t> pos((size_t)loc[nsub], 0);
+        parallel_for(nsub, [&](int i) {
+            const HostSub& h = s->hs[i];
+            const int nl = h.n_local(), T = Ts[i];
+            for (int k = 0; k < nl; ++k) {
+                const int p = h.pin[k < T ? lev[0][i].rhs_row[k] : k];
+                pin[loc[i] + k] = p;
+                gin[loc[i] + k] = (int32_t)(p < h.n_owned ? h.begin + p : h.ghosts[p - h.n_owned]);
+                const int q = h.pout[k];
+                gout[loc[i] + k] = q < T ? lev[1][i].pos[q] : q;
+            }
+            for (int k = 0; k < T; ++k) {
+                u2l[loc[i] + k] = lev[1][i].rhs_row[k];
+                pos[loc[i] + k] = (uint16_t)lev[0][i].pos[k];
+            }
+        });
+        RET_IF(upload(s, &y.gin, gin));
+        RET_IF(upload(s, &y.pin, pin));
+        RET_IF(upload(s, &y.u2l, u2l));
+        RET_IF(upload(s, &y.gout, gout));
+        RET_IF(upload(s, &y.pos, pos));
+        for (int f = 0; f < 2; ++f) {
+            std::vector<LevelSweep>& q = lev[f];
+            // offsets of the subdomains in the concatenated arrays
+            std::vector<int64_t> s0(nsub + 1, 0), t0(nsub + 1, 0), o0(nsub + 1, 0), w0(nsub + 1, 0), b0(nsub + 1, 0);
+            for (int i = 0; i < nsub; ++i) {
+                s0[i + 1] = s0[i] + (int64_t)q[i].val.size() / 128;
+                t0[i + 1] = t0[i] + (int64_t)q[i].task.size();
+                o0[i + 1] = o0[i] + (int64_t)q[i].bout.size();
+                w0[i + 1] = w0[i] + (int64_t)q[i].wsrc.size();
+                b0[i + 1] = b0[i] + (int64_t)q[i].bk.size();
+            }
+            std::vector<unsigned char> ent((size_t)s0[nsub] * sb);
+            std::vector<uint4> task((size_t)t0[nsub]);
+            std::vector<LevelWarp> warp((size_t)nsub * nw);
+            std::vector<uint16_t> rslot((size_t)loc[nsub], 0), bout((size_t)o0[nsub]);
+            std::vector<double> dinv((size_t)loc[nsub], 1.0);
+            std::vector<int32_t> src, dsrc, bk;
+            std::vector<int64_t> boff, wsrc, wpos;
+            if (track) {
+                src.resize((size_t)s0[nsub] * 128);
+                dsrc.assign((size_t)loc[nsub], -1);
+                bk.resize((size_t)b0[nsub]);
+                boff.resize((size_t)b0[nsub] + 1, w0[nsub]);
+                wsrc.resize((size_t)w0[nsub]);
+                wpos.resize((size_t)w0[nsub]);
+            }
+            parallel_for(nsub, [&](int i) {
+                LevelSweep& x = q[i];
+                for (int64_t st = 0; st < s0[i + 1] - s0[i]; ++st) {
+                    unsigned char* p = ent.data() + (size_t)(s0[i] + st) * sb;
+                    for (int e = 0; e < 128; ++e) {
+                        const double val = x.val[(size_t)(128 * st + e)];
+                        if (rs == 4) reinterpret_cast<float*>(p)[e] = (float)val;
+                        else reinterpret_cast<double*>(p)[e] = val;
+                        reinterpret_cast<uint16_t*>(p + 128 * rs)[e] = (uint16_t)x.col[(size_t)(128 * st + e)];
+                    }
+                }
+                for (size_t t = 0; t < x.task.size(); ++t) {
+                    task[(size_t)t0[i] + t] = x.task[t];
+                    if (x.task[t].x & S2L_LTASK_NO_RHS) task[(size_t)t0[i] + t].z += (uint32_t)o0[i];
+                }
+                std::copy(x.bout.begin(), x.bout.end(), bout.begin() + o0[i]);
+                for (int w = 0; w < nw; ++w) {
+                    LevelWarp u{};
+                    u.step = s0[i] + x.wstep[w];
+                    u.nstep = (int)(x.wstep[w + 1] - x.wstep[w]);
+                    u.task = t0[i] + x.wtask[w];
+                    u.ntask = (int)(x.wtask[w + 1] - x.wtask[w]);
+                    u.lo = loc[i];
+                    u.rhs = x.n0 + (int)x.wrhs[w];
+                    u.nrhs = (int)(x.wrhs[w + 1] - x.wrhs[w]);
+                    u.n0 = x.n0;
+                    u.nst = x.nst;
+                    u.T = Ts[i];
+                    warp[(size_t)i * nw + w] = u;
+                }
+                for (int k = 0; k < Ts[i]; ++k) {
+                    rslot[loc[i] + k] = (uint16_t)x.pos[x.rhs_row[k]];
+                    dinv[loc[i] + k] = x.dinv[k];
+                    if (track) dsrc[loc[i] + k] = x.dsrc[k];
+                }
+                if (track) {
+                    std::copy(x.src.begin(), x.src.end(), src.begin() + 128 * s0[i]);
+                    std::copy(x.bk.begin(), x.bk.end(), bk.begin() + b0[i]);
+                    for (size_t b = 0; b < x.bk.size(); ++b) boff[(size_t)b0[i] + b] = w0[i] + x.boff[b];
+                    for (size_t e = 0; e < x.wsrc.size(); ++e) {
+                        wsrc[(size_t)w0[i] + e] = x.wsrc[e] >= 0 ? fb[i] + x.wsrc[e] : -1;
+                        wpos[(size_t)w0[i] + e] = 128 * s0[i] + x.wpos[e];
+                    }
+                }
+            });
+            for (int i = 0; i < nsub && v == 0; ++i) {
+                const LevelSweep& x = q[i];
+                s->st_levels_max = std::max<int64_t>(s->st_levels_max, x.nlev);
+                s->st_levels_sum += x.nlev;
+                s->st_sparse_nnz += x.real;
+                s->st_pad += (int64_t)x.val.size() - x.real;
+                s->st_tasks += (int64_t)x.task.size();
+                s->st_blocks += x.nblk;
+                // algorithmic bytes: the entries with their columns, 1/diag and the task descriptors
+                bytes += (double)x.real * (rs + 2) + (double)Ts[i] * rs + (double)x.task.size() * 16;
+            }
+            RET_IF(upload(s, &y.ent[f], ent));
+            RET_IF(upload(s, &y.task[f], task));
+            RET_IF(upload(s, &y.warp[f], warp));
+            RET_IF(upload(s, &y.rslot[f], rslot));
+            RET_IF(upload(s, &y.bout[f], bout));
+            if (rs == 4) RET_IF(upload_real<float>(s, &y.dinv[f], dinv));
+            else RET_IF(upload_real<double>(s, &y.dinv[f], dinv));
+            if (track) {
+                y.nblk[f] = (int64_t)bk.size();
+                RET_IF(upload(s, &y.src[f], src));
+                RET_IF(upload(s, &y.dsrc[f], dsrc));
+                RET_IF(upload(s, &y.bk[f], bk));
+                RET_IF(upload(s, &y.boff[f], boff));
+                RET_IF(upload(s, &y.wsrc[f], wsrc));
+                RET_IF(upload(s, &y.wpos[f], wpos));
+            }
+            CUDA_OK(s, cudaStreamSynchronize(s->setup_stream));
+            q.clear();
+        }
+        s->nlay = v + 1;
+        return S2L_OK;
+    };
+    for (int v = 0; v < nlay; ++v) {
+        const size_t mark = s->allocs.size(), before = s->bytes;
+        const int rc = build(v);
+        if (rc == S2L_OK) continue;
+        if (v == 0 || (rc != S2L_ERR_OOM && rc != S2L_ERR_STATE)) return rc;
+        // no memory for a second layout: blocks run on the first
+        CUDA_OK(s, cudaStreamSynchronize(s->setup_stream));
+        for (size_t i = mark; i < s->allocs.size(); ++i) cudaFree(s->allocs[i]);
+        s->allocs.resize(mark);
+        std::lock_guard<std::mutex> g(s->ctx->mu);
+        s->ctx->used -= std::min(s->ctx->used, s->bytes - before);
+        s->bytes = before;
+        s->lay[1] = {};
+    }
+    s->solve_bytes = bytes;
+    return S2L_OK;
+}
+
 int check_ready(s2l_setup* s)
 {
     if (!s) return S2L_ERR_BADARG;
@@ -1135,7 +1367,13 @@ struct Prof {
 
 // ------------------------------------------------------------------------------ solve-phase pieces
 template <typename Real>
-LocalSolveArgs<Real> solve_args(s2l_work* w)
+LevelFactor<Real> level_factor(const s2l_setup::LevelLay& y, int f)
+{
+    return {y.ent[f], (const Real*)y.dinv[f], y.rslot[f], y.task[f], y.warp[f], y.bout[f], y.pos};
+}
+
+template <typename Real>
+LocalSolveArgs<Real> solve_args(s2l_work* w, int K, int mode)
 {
     s2l_setup* s = w->s;
     LocalSolveArgs<Real> a{};
@@ -1146,6 +1384,20 @@ LocalSolveArgs<Real> solve_args(s2l_work* w)
                   s->d_bfirst[f], s->d_boff[f],            s->d_bioff[f],             s->d_bslot[f],
                   (const Real*)s->d_binv[f]};
     a.u2l = s->d_u2l;
+    a.gout = s->d_gout;
+    a.gather = mode == 2 ? s->d_pin : s->d_gin;
+    a.K = K;
+    a.KC = std::min(K, s->kc_max);
+    if (s->nlay > 0) {
+        const auto& y = s->lay[K > 1 ? s->nlay - 1 : 0];
+        for (int f = 0; f < 2; ++f) a.lf[f] = level_factor<Real>(y, f);
+        a.cs = y.cs;
+        a.slots = y.slots;
+        a.u2l = y.u2l;
+        a.gout = y.gout;
+        a.gather = mode == 2 ? y.pin : y.gin;
+        a.KC = std::min(K, y.kc_max);
+    }
     a.tr_sub = s->d_tr_sub;
     a.tr_i = s->d_tr_i;
     a.lts_ptr = s->d_lts_ptr;
@@ -1159,14 +1411,11 @@ LocalSolveArgs<Real> solve_args(s2l_work* w)
     a.uu = s->d_uu;
     a.linv = (const Real*)s->d_linv;
     a.uinv = (const Real*)s->d_uinv;
-    a.gout = s->d_gout;
     a.ylocal = w->d_ylocal;
     a.ybuf = (Real*)w->d_ybuf;
     a.xbuf = (Real*)w->d_xbuf;
     a.gflags = w->d_gflags;
     a.err = w->d_err;
-    a.K = 1;
-    a.KC = 1;
     a.nloc = s->nloc;
     a.spin_limit = s->opt_spin_limit.load();
     a.spin_sleep_ns = s->opt_spin_sleep.load();
@@ -1260,18 +1509,16 @@ int run_local_solve(s2l_work* w, const double* in, const double* base, double* o
     int launched = 0;
     const size_t smem = w->d_gflags ? 0 : s->smem_bytes;
     if (s->real == S2L_REAL_F32) {
-        LocalSolveArgs<float> a = solve_args<float>(w);
+        LocalSolveArgs<float> a = solve_args<float>(w, 1, mode);
         a.sub_list = sub_list;
-        a.gather = mode == 2 ? s->d_pin : s->d_gin;
         a.in = mode == 2 ? local_in : in;
         a.base = base;
         a.out = out;
         a.mode = mode;
         e = launch_local_solve<float>(w->stream, a, nb, smem, tr0, trn, us0, usn, &launched);
     } else {
-        LocalSolveArgs<double> a = solve_args<double>(w);
+        LocalSolveArgs<double> a = solve_args<double>(w, 1, mode);
         a.sub_list = sub_list;
-        a.gather = mode == 2 ? s->d_pin : s->d_gin;
         a.in = mode == 2 ? local_in : in;
         a.base = base;
         a.out = out;
@@ -1421,8 +1668,7 @@ int local_solve_block_t(s2l_work* w, int K, const double* in, const double* base
 {
     s2l_setup* s = w->s;
     s2l_work::Block& B = w->blk;
-    LocalSolveArgs<Real> a = solve_args<Real>(w);
-    a.gather = s->d_gin;
+    LocalSolveArgs<Real> a = solve_args<Real>(w, K, mode);
     a.in = in;
     a.base = base;
     a.out = out;
@@ -1431,8 +1677,7 @@ int local_solve_block_t(s2l_work* w, int K, const double* in, const double* base
     a.ybuf = (Real*)B.ybuf;
     a.xbuf = (Real*)B.xbuf;
     a.gflags = B.gflags;
-    a.K = K;
-    a.KC = B.gflags ? 1 : std::min(K, s->kc_max);
+    if (B.gflags) a.KC = 1;
     const size_t smem = B.gflags ? 0 : sweep_smem(s, a.KC);
     int launched = 0;
     const cudaError_t e = launch_local_solve<Real>(w->stream, a, s->nsub, smem, 0, s->tr_first_h[s->nsub], 0,
@@ -2406,11 +2651,24 @@ int s2l_gpu_setup_end(s2l_setup* s)
     tm.force_rows = s->opt_tail_rows;
     tm.tail_min = s->opt_tail_min;
     tm.tail_max = s->opt_tail_max;
-    tm.hop_s = s->opt_hop_us * 1e-6;
+    // Level sweeps, unless the chain blocks are off: without blocks the levels are single rows by the
+    // hundred and a barrier for each costs more than the dataflow sweeps' flags.  (The layouts below
+    // still fall back to dataflow sweeps when x and s do not fit the shared memory.)
+    bool level = s->local_kind == 0 && s->opt_chain > 1 && s->opt_level != 0;
+    const int lcap = std::min(8 * s->opt_chain, S2L_LEVEL_CAP);
     tm.bw = s->opt_bw_gbs * 1e9;
     tm.nsub = nsub;
     tm.real_bytes = (double)rs;
-    tm.chain = s->opt_chain;
+    // the tail split's model of the sweeps
+    auto sweep_model = [&](bool lv, int ring) {
+        tm.hop_s = (s->opt_hop_us > 0.0 ? s->opt_hop_us : lv ? S2L_LEVEL_HOP_US : 0.25) * 1e-6;
+        tm.chain = lv ? lcap : s->opt_chain;
+        tm.fold = !lv;
+        tm.index_bytes = lv ? 2.0 : 4.0;
+        // shared memory: x and ready flags, or x, some s and a ring of `ring` steps per warp
+        tm.slot_bytes = lv ? rs : rs + 1.0;
+        tm.smem_cap = (double)S2L_SWEEP_SMEM_CAP - (lv ? (double)level_smem_bytes(rs, 1024, 1, ring) : 0.0);
+    };
     // per subdomain and independent of the others: on several host threads
     std::vector<char> ldlt_bad(nsub, 0);
     parallel_for(nsub, [&](int i) {
@@ -2444,10 +2702,42 @@ int s2l_gpu_setup_end(s2l_setup* s)
                 }
             }
         }
-        Ts[i] = choose_tail(h.L, Us[i], nl, tm);
     });
     for (int i = 0; i < nsub; ++i)
         if (ldlt_bad[i]) return s->fail(S2L_ERR_BADARG, "LDLT: L must store its unit diagonal");
+    std::vector<int> levels(nsub, 0);
+    int deepest = 0;  // levels of the split's deepest subdomain
+    auto fits = [&]() {
+        bool ok = true;
+        for (int i = 0; i < nsub; ++i) ok = ok && (double)Ts[i] * tm.slot_bytes + 64.0 <= tm.smem_cap;
+        return ok;
+    };
+    auto split = [&](bool lv, int ring) {  // false: a sparse part too large for level sweeps with such a ring
+        sweep_model(lv, ring);
+        parallel_for(nsub, [&](int i) {
+            if (!s->hs[i].amg) Ts[i] = choose_tail(s->hs[i].L, Us[i], s->hs[i].n_local(), tm, &levels[i]);
+        });
+        deepest = *std::max_element(levels.begin(), levels.end());
+        return !lv || fits();
+    };
+    // rings of four steps keep the loads ahead (bubbles3d 100^3 / 64, FP64: 1094 us a local solve with
+    // three, 1630 with two)
+    split(false, 0);
+    // Few levels stay with the flags: a hand-over costs both about the same (1 us), but a level sweep's
+    // stages come twice a level, and the longer tail that its split takes costs what the shorter chain
+    // saves.  Local solves in us, dataflow and level sweeps: 16 levels (bubbles3d 24^3 / 8) 68 and 76,
+    // 23 (40^3 / 32) 138 and 158, 24 (32^3 / 8) 124 and 139, 32 (36^3 / 8) 199 and 170, 40 (40^3 / 8)
+    // 275 and 205, 63 (convdiff3d 32^3 / 12) 262 and 157, 77 (poisson2d 200^2 / 8) 224 and 117.
+    if (level) {
+        const std::vector<int> dataflow = Ts;
+        const int flags = deepest;
+        level = (s->opt_level == 1 || flags > 28) && (split(true, 4) || split(true, 2));
+        // A refactorization's time goes by its longest sparse part and its dense tails: it keeps the
+        // split of the dataflow sweeps (bubbles3d 40^3 / 8: 46.7 ms, 49 to 53 with the level sweeps' own)
+        const std::vector<int> own = Ts;
+        if (!level || s->opt_refactor) Ts = dataflow;
+        if (level && !fits()) Ts = own;
+    }
     s->sweep_group = s->opt_group ? s->opt_group : 16;  // widest lane group of a sweep row
     const int nw = S2L_BS_SWEEP / 32;
     // pass 2: layouts
@@ -2471,6 +2761,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
     s->uu_first_h.assign(nsub + 1, 0);
     double bytes = 0.0;
     int max_T = 0, max_nl = 0;
+    for (int i = 0; i < nsub; ++i) max_T = std::max(max_T, Ts[i]);
     int64_t sparse_nnz = 0;
     // refactorization plan (host side; see RefactorArgs)
     const bool rfon = s->opt_refactor != 0;
@@ -2523,6 +2814,28 @@ int s2l_gpu_setup_end(s2l_setup* s)
                     q.mposU[e] = llt ? q.P.find(c, r) : q.P.find(r, c);
                 }
         }
+    });
+    for (int i = 0; i < nsub; ++i)
+        if (pre[i].code != S2L_OK) return s->fail(pre[i].code, "subdomain " + std::to_string(i) + ": " + pre[i].err);
+    if (level) {
+        const int rc = build_level_layouts(s, Us, Ts, [&](int i, int f) -> const std::vector<int32_t>* {
+            return !rfon ? nullptr : f == 0 ? &pre[i].mposL : &pre[i].mposU;
+        }, [&](int i) { return (int64_t)pre[i].P.ri.size(); }, lcap);
+        if (rc == S2L_ERR_STATE) {  // no room for x and s: dataflow sweeps
+            level = false;
+            split(false, 0);
+            max_T = *std::max_element(Ts.begin(), Ts.end());
+        } else if (rc != S2L_OK) {
+            return rc;
+        }
+    }
+    if (!level) parallel_for(nsub, [&](int i) {
+        HostSub& h = s->hs[i];
+        if (h.amg) return;
+        PreLayout& q = pre[i];
+        const HostCsr& U = Us[i];
+        const int T = Ts[i];
+        const bool unitL = h.kind != S2L_FACTOR_LLT;
         build_sweep(h.L, T, true, unitL, nw, s->sweep_group, s->opt_epl, s->opt_chain, q.sl, q.err, rfon ? &q.mposL : nullptr);
         if (q.err.empty())
             build_sweep(U, T, false, false, nw, s->sweep_group, s->opt_epl, s->opt_chain, q.su, q.err, rfon ? &q.mposU : nullptr);
@@ -2568,7 +2881,6 @@ int s2l_gpu_setup_end(s2l_setup* s)
         const bool unitL = h.kind != S2L_FACTOR_LLT;
         const int T = Ts[i];
         const int sz = nl - T;
-        max_T = std::max(max_T, T);
         Sweep& sl = pre[i].sl;
         Sweep& su = pre[i].su;
         const FPat& P = pre[i].P;
@@ -2670,9 +2982,11 @@ int s2l_gpu_setup_end(s2l_setup* s)
             }
             rf_fbase.push_back(fb + (int64_t)P.ri.size());
         }
-        s->st_levels_max = std::max<int64_t>(s->st_levels_max, std::max(sl.nlev, su.nlev));
-        s->st_levels_sum += sl.nlev + su.nlev;
-        for (int f = 0; f < 2; ++f) {
+        if (!level) {
+            s->st_levels_max = std::max<int64_t>(s->st_levels_max, std::max(sl.nlev, su.nlev));
+            s->st_levels_sum += sl.nlev + su.nlev;
+        }
+        for (int f = 0; f < 2 && !level; ++f) {
             const Sweep& q = f == 0 ? sl : su;
             const int64_t e0 = sw_col[f].size(), t0 = sw_thdr[f].size(), s0 = sw_tslot[f].size();
             for (int w = 0; w < nw; ++w) {
@@ -2717,8 +3031,10 @@ int s2l_gpu_setup_end(s2l_setup* s)
             bytes += (double)q.blk_inv.size() * rs + (double)q.blk_slot.size() * 4 + (double)(q.blk_off.size() - 1) * 16;
         }
         // backward slot -> forward slot
-        for (int u = 0; u < T; ++u) u2l.push_back(sl.pos[su.order[u]]);
-        u2l.resize(u2l.size() + sz, 0);
+        if (!level) {
+            for (int u = 0; u < T; ++u) u2l.push_back(sl.pos[su.order[u]]);
+            u2l.resize(u2l.size() + sz, 0);
+        }
         // L coupling of the tail rows (columns as forward slots) and the dense lower tail
         s->tr_first_h[i] = (int)tr_sub.size();
         if (sz > 0) {
@@ -2729,7 +3045,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
                 for (int64_t e = h.L.rp[k]; e < h.L.rp[k + 1]; ++e) {
                     const int c = h.L.ci[e];
                     if (c < T) {
-                        lts_col.push_back(sl.pos[c]);
+                        lts_col.push_back(level ? c : sl.pos[c]);
                         lts_val.push_back(h.L.v[e]);
                         if (rfon) rf_lts.push_back(fb + P.find(k, c));
                     } else if (c < k) {
@@ -2776,7 +3092,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
                         if (rfon) rf_ust.push_back(fb + (llt ? P.find(U.ci[e], r) : P.find(r, U.ci[e])));
                     }
                 us_sub.push_back(i);
-                us_r.push_back(sl.pos[r]);
+                us_r.push_back(level ? r : sl.pos[r]);
                 ust_ptr.push_back((int64_t)ust_col.size());
             }
             for (size_t k = 0; k < rows.size();) {
@@ -2802,13 +3118,14 @@ int s2l_gpu_setup_end(s2l_setup* s)
             const int64_t g = j < h.n_owned ? h.begin + j : h.ghosts[j - h.n_owned];
             l2g.push_back((int32_t)g);
         }
-        // forward gather per slot (< T) or tail row (>= T); backward output position per local j
-        for (int k = 0; k < nl; ++k) {
+        // forward gather per slot (< T) or tail row (>= T); backward output position per local j (the level
+        // sweeps' layouts have their own)
+        for (int k = 0; k < nl && !level; ++k) {
             const int prow = k < T ? sl.order[k] : k;
             gin.push_back(l2g[loc + h.pin[prow]]);
             pin.push_back(h.pin[prow]);
         }
-        for (int j = 0; j < nl; ++j) {
+        for (int j = 0; j < nl && !level; ++j) {
             const int q = h.pout[j];
             gout.push_back(q < T ? su.pos[q] : q);
         }
@@ -2823,12 +3140,13 @@ int s2l_gpu_setup_end(s2l_setup* s)
     s->uu_first_h[nsub] = (int)uu.size();
     uu.push_back((int32_t)us_sub.size());  // the end of the last unit
     s->nloc = loc;
-    s->st_sparse_nnz = sparse_nnz;
+    if (!level) s->st_sparse_nnz = sparse_nnz;
     s->st_coupling_nnz = (int64_t)lts_col.size() + (int64_t)ust_col.size();
     s->st_dense_entries = d_off[nsub];
     s->st_tail_rows = (int64_t)tr_sub.size();
     bytes += (double)s->st_coupling_nnz * (rs + 4) + (double)(tr_sub.size() + us_sub.size()) * (8 + 8 + rs);
-    for (int f = 0; f < 2; ++f) {
+    if (level) bytes += s->solve_bytes;  // (the sparse parts of build_level_layouts)
+    for (int f = 0; f < 2 && !level; ++f) {
         sw_wtask[f].push_back((int64_t)sw_thdr[f].size());
         sw_wslot[f].push_back((int64_t)sw_tslot[f].size());
         sw_went[f].push_back((int64_t)sw_col[f].size());
@@ -3155,6 +3473,10 @@ int s2l_gpu_setup_end(s2l_setup* s)
         s->smem_bytes = 0;
         s->need_gflags = true;
     }
+    if (level) {
+        s->smem_bytes = level_smem_bytes(rs, s->lay[0].slots, 1, level_ring(rs, s->lay[0].slots, 1));
+        s->need_gflags = false;
+    }
     s->max_nl = max_nl;
     s->max_T = max_T;
     s->kc_max = 1;
@@ -3162,6 +3484,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
         for (int kc = 2; kc <= 4; kc *= 2)
             if ((((slots * kc * rs) + 15) & ~(size_t)15) + ((slots + 15) & ~(size_t)15) <= smem_cap)
                 s->kc_max = kc;
+    if (level) s->kc_max = s->lay[s->nlay - 1].kc_max;
     CUDA_OK(s, cudaStreamSynchronize(s->setup_stream));
     // host staging no longer needed
     s->A.ci = {};  // the row pointers stay: s2l_gpu_update_matrix recomputes the row sums with them
@@ -3314,7 +3637,17 @@ int refactor_commit_factors(s2l_setup* s, cudaStream_t st)
 {
     auto& R = s->rf;
     const int nsub = s->nsub;
-    for (int f = 0; f < 2; ++f) {
+    for (int v = 0; v < s->nlay; ++v) {
+        auto& y = s->lay[v];
+        const int wps = y.cs * (S2L_BS_LEVEL / 32);
+        for (int f = 0; f < 2; ++f) {
+            launch_refactor_dinv<Real>(st, nsub, s->d_subs, R.fbase, R.F, y.dsrc[f], (Real*)y.dinv[f]);
+            launch_refactor_level_values<Real>(st, nsub * wps, wps, R.fbase, R.F, level_factor<Real>(y, f), y.src[f],
+                                               y.dsrc[f], y.ent[f]);
+            launch_refactor_level_blocks<Real>(st, y.nblk[f], y.bk[f], y.boff[f], y.wsrc[f], y.wpos[f], R.F, y.ent[f]);
+        }
+    }
+    for (int f = 0; f < 2 && s->nlay == 0; ++f) {
         launch_refactor_dinv<Real>(st, nsub, s->d_subs, R.fbase, R.F, R.sw_dsrc[f], (Real*)s->d_dinv[f]);
         launch_refactor_sweep_values<Real>(st, nsub, R.fbase, R.F, s->d_wtask[f], s->d_wslot[f], s->d_went[f],
                                            s->d_thdr[f], s->d_tslot[f], R.sw_src[f], s->d_subs, R.sw_dsrc[f],
@@ -3554,6 +3887,10 @@ int s2l_gpu_setup_option(s2l_setup* s, const char* name, double value)
         const int c = (int)value;
         if (c < 1 || c > S2L_CHAIN_MAX) return s->fail(S2L_ERR_BADARG, "chain_block must be in [1, 16]");
         s->opt_chain = c;
+    } else if (n == "level_sweeps") {
+        const int v = (int)value;
+        if (v < -1 || v > 1) return s->fail(S2L_ERR_BADARG, "level_sweeps must be -1, 0 or 1");
+        s->opt_level = v;
     } else if (n == "refactor") {
         s->opt_refactor = value != 0.0;
     } else if (n == "amg_single") {
@@ -3575,6 +3912,7 @@ int s2l_gpu_setup_stat(const s2l_setup* s, const char* name, double* value)
     else if (n == "tail_rows") *value = (double)s->st_tail_rows;
     else if (n == "sweep_group") *value = (double)s->sweep_group;
     else if (n == "smem_bytes") *value = (double)s->smem_bytes;
+    else if (n == "level_sweeps") *value = (double)(s->nlay > 0 ? s->lay[0].cs : 0);
     else if (n == "levels_max") *value = (double)s->st_levels_max;
     else if (n == "chain_blocks") *value = (double)s->st_blocks;
     else if (n == "sweep_tasks") *value = (double)s->st_tasks;

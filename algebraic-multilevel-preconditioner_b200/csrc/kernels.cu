@@ -1617,7 +1617,10 @@ cudaError_t launch_local_solve_k(cudaStream_t st, const LocalSolveArgs<Real>& a,
 {
     cudaError_t e;
     const int grid = nblocks * (K / KC);
-    if (smem > 0) {
+    if (a.cs > 0) {
+        e = launch_level_sweep<Real>(st, a, true, nblocks);
+        if (e != cudaSuccess) return e;
+    } else if (smem > 0) {
         // the limit is a process-wide attribute of the kernel: always the same cap, so launches of
         // setups with different shared-memory sizes from several threads cannot undercut each other
         if (smem > S2L_SWEEP_SMEM_CAP) return cudaErrorInvalidValue;
@@ -1643,7 +1646,10 @@ cudaError_t launch_local_solve_k(cudaStream_t st, const LocalSolveArgs<Real>& a,
         sparse_coupling_kernel<Real, K><<<(uu_count + 7) / 8, 256, 0, st>>>(a, uu_first, uu_count);
         nl += 1;
     }
-    if (smem > 0)
+    if (a.cs > 0) {
+        e = launch_level_sweep<Real>(st, a, false, nblocks);
+        if (e != cudaSuccess) return e;
+    } else if (smem > 0)
         sweep_kernel<Real, true, false, KC><<<grid, S2L_BS_SWEEP, smem, st>>>(a);
     else
         sweep_kernel<Real, false, false, KC><<<grid, S2L_BS_SWEEP, 0, st>>>(a);
@@ -1656,7 +1662,7 @@ cudaError_t launch_local_solve(cudaStream_t st, const LocalSolveArgs<Real>& a, i
                                int tr_count, int uu_first, int uu_count, int* launches)
 {
     // (KC, K): right-hand sides per sweep CTA and in all; the setup's shared memory fixes KC
-    const int K = a.K, KC = smem > 0 ? a.KC : 1;
+    const int K = a.K, KC = a.cs > 0 || smem > 0 ? a.KC : 1;
 #define S2L_LS(KC_, K_)                                                                                         \
     if (KC == KC_ && K == K_)                                                                                  \
     return launch_local_solve_k<Real, KC_, K_>(st, a, nblocks, smem, tr_first, tr_count, uu_first, uu_count, \

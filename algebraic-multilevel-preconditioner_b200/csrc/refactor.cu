@@ -398,6 +398,80 @@ __global__ void __launch_bounds__(256) sweep_values_kernel(int nsub, const int64
     }
 }
 
+// place of value e (128 per step) in the steps of the level sweeps
+template <typename Real>
+__device__ __forceinline__ Real* level_value(unsigned char* ent, int64_t e)
+{
+    return reinterpret_cast<Real*>(ent + (e >> 7) * level_step_bytes(sizeof(Real))) + (e & 127);
+}
+
+// values of the level sweeps: one warp per warp of the sweep walking its tasks; entry value = F(src),
+// of a single row / its diagonal (padding 0, entries of W^-1 skipped)
+template <typename Real>
+__global__ void __launch_bounds__(256) level_values_kernel(int nwarps, int warps_per_sub,
+                                                           const int64_t* __restrict__ fbase,
+                                                           const double* __restrict__ F, const LevelFactor<Real> lf,
+                                                           const int32_t* __restrict__ src,
+                                                           const int32_t* __restrict__ dsrc,
+                                                           unsigned char* __restrict__ ent)
+{
+    const int wi = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
+    if (wi >= nwarps) return;
+    const int sid = wi / warps_per_sub;
+    const int64_t fb = fbase[sid];
+    const LevelWarp w = lf.warp[wi];
+    int64_t eo = w.step * 128, rp = w.lo + w.rhs;
+    for (int64_t t = w.task; t < w.task + w.ntask; ++t) {
+        const uint4 d = lf.task[t];
+        const int R = (int)((d.x >> 3) & 63u), k = lane >> (int)(d.x & 7u);
+        const bool rhs = !(d.x & S2L_LTASK_NO_RHS);
+        double di = 1.0;  // 1 / diagonal of a single row, in FP64 as at setup
+        if (rhs && k < R) {
+            const int32_t q = dsrc[rp + k];
+            if (q >= 0) di = 1.0 / F[fb + q];
+        }
+        const int64_t e1 = eo + (int64_t)(d.y >> 16) * 128;
+        for (eo += lane; eo < e1; eo += 32) {
+            const int32_t p = src[eo];
+            if (p >= 0) *level_value<Real>(ent, eo) = (Real)(F[fb + p] * di);
+            else if (p == -1) *level_value<Real>(ent, eo) = Real(0);
+        }
+        eo = e1;
+        if (rhs) rp += R;
+    }
+}
+
+// diagonal blocks of the level sweeps: W from F, W^-1 by forward substitution (as at setup), a
+// thread per column, and its entries to their places; one CTA per block
+template <typename Real>
+__global__ void __launch_bounds__(S2L_LEVEL_CAP) level_blocks_kernel(const int32_t* __restrict__ bk,
+                                                                     const int64_t* __restrict__ boff,
+                                                                     const int64_t* __restrict__ wsrc,
+                                                                     const int64_t* __restrict__ wpos,
+                                                                     const double* __restrict__ F,
+                                                                     unsigned char* __restrict__ ent)
+{
+    __shared__ double W[S2L_LEVEL_CAP * (S2L_LEVEL_CAP + 1) / 2], X[S2L_LEVEL_CAP * (S2L_LEVEL_CAP + 1) / 2];
+    const int k = bk[blockIdx.x], np = k * (k + 1) / 2;
+    const int64_t o = boff[blockIdx.x];
+    for (int i = 0; i < k; ++i)
+        for (int j = threadIdx.x; j <= i; j += S2L_LEVEL_CAP) {
+            const int64_t q = wsrc[o + i * (i + 1) / 2 + j];
+            W[i * (i + 1) / 2 + j] = q >= 0 ? F[q] : (i == j ? 1.0 : 0.0);
+        }
+    __syncthreads();
+    const int j = threadIdx.x;
+    if (j < k)
+        for (int i = j; i < k; ++i) {
+            double v = i == j ? 1.0 : 0.0;
+            for (int p = j; p < i; ++p) v -= W[i * (i + 1) / 2 + p] * X[p * (p + 1) / 2 + j];
+            X[i * (i + 1) / 2 + j] = v / W[i * (i + 1) / 2 + i];
+        }
+    __syncthreads();
+    for (int e = threadIdx.x; e < np; e += S2L_LEVEL_CAP) *level_value<Real>(ent, wpos[o + e]) = (Real)X[e];
+}
+
 // 1 / diagonal per slot (1 where the source is -1: unit diagonals, chain-block rows, tail rows)
 template <typename Real>
 __global__ void dinv_kernel(int nsub, const DevSub* __restrict__ subs, const int64_t* __restrict__ fbase,
@@ -670,6 +744,23 @@ void launch_refactor_blocks(cudaStream_t st, int64_t nblocks, const int64_t* bof
 }
 
 template <typename Real>
+void launch_refactor_level_values(cudaStream_t st, int nwarps, int warps_per_sub, const int64_t* fbase, const double* F,
+                                  const LevelFactor<Real>& lf, const int32_t* src, const int32_t* dsrc,
+                                  unsigned char* ent)
+{
+    if (nwarps > 0)
+        level_values_kernel<Real><<<(nwarps + 7) / 8, 256, 0, st>>>(nwarps, warps_per_sub, fbase, F, lf, src, dsrc, ent);
+}
+
+template <typename Real>
+void launch_refactor_level_blocks(cudaStream_t st, int64_t nblocks, const int32_t* bk, const int64_t* boff,
+                                  const int64_t* wsrc, const int64_t* wpos, const double* F, unsigned char* ent)
+{
+    if (nblocks > 0)
+        level_blocks_kernel<Real><<<(unsigned)nblocks, S2L_LEVEL_CAP, 0, st>>>(bk, boff, wsrc, wpos, F, ent);
+}
+
+template <typename Real>
 void launch_gather_values(cudaStream_t st, int64_t count, const int64_t* src, const double* F, Real* out)
 {
     if (count > 0) gather_values_kernel<Real><<<grid_for(count, 256), 256, 0, st>>>(count, src, F, out);
@@ -720,7 +811,17 @@ template void launch_refactor_blocks<float>(cudaStream_t, int64_t, const int64_t
                                             const uint8_t*, const int64_t*, const double*, float*, float*);
 template void launch_tail_inverses<double>(cudaStream_t, const double*, const double*, int, int, double*, double*);
 template void launch_tail_inverses<float>(cudaStream_t, const double*, const double*, int, int, float*, float*);
+template void launch_refactor_level_values<double>(cudaStream_t, int, int, const int64_t*, const double*,
+                                                   const LevelFactor<double>&, const int32_t*, const int32_t*,
+                                                   unsigned char*);
+template void launch_refactor_level_blocks<double>(cudaStream_t, int64_t, const int32_t*, const int64_t*, const int64_t*,
+                                                   const int64_t*, const double*, unsigned char*);
 template void launch_gather_values<double>(cudaStream_t, int64_t, const int64_t*, const double*, double*);
+template void launch_refactor_level_values<float>(cudaStream_t, int, int, const int64_t*, const double*,
+                                                   const LevelFactor<float>&, const int32_t*, const int32_t*,
+                                                   unsigned char*);
+template void launch_refactor_level_blocks<float>(cudaStream_t, int64_t, const int32_t*, const int64_t*, const int64_t*,
+                                                   const int64_t*, const double*, unsigned char*);
 template void launch_gather_values<float>(cudaStream_t, int64_t, const int64_t*, const double*, float*);
 
 }  // namespace s2l

@@ -35,6 +35,13 @@
 #define S2L_SPIN_SLEEP_NS 0   // pause of a sweep warp after a poll that found a column not ready (ns; 0 = none)
 #endif
 #define S2L_SPIN_LIMIT (1 << 24)  // polls of one ready flag before a sweep gives up (error 1)
+#define S2L_BS_LEVEL 512      // threads of a CTA of the level sweeps (level_sweep.cu)
+#define S2L_LEVEL_HOP_US 2.0  // the tail split's time of a level of a level sweep (hop_us default)
+#define S2L_LEVEL_CAP 64      // rows of a block of the level sweeps, at most
+#define S2L_LEVEL_CS 8        // CTAs (a cluster) per subdomain of the level sweeps, at most
+#define S2L_LTASK_TO_S 512u     // task flags of the level sweeps (LevelFactor): the results are s of a block,
+                                // for the CTA in bits 12-15 (else x, for all)
+#define S2L_LTASK_NO_RHS 1024u  // x of block rows: the sums themselves (else right-hand side - sum)
 #define S2L_GS_SMEM_CAP (224 * 1024)  // shared memory of a Gauss-Seidel sweep CTA (its subdomain's x)
 
 struct DevSub {
@@ -78,8 +85,41 @@ struct SweepFactor {
     const Real* blk_inv;
 };
 
+// The same sparse part in the layout of the level sweeps (level_layout.inl): per warp of the
+// subdomain's cluster a list of tasks in stage order and one stream of their steps.  A task is R rows
+// with G lanes each; a step holds four entries per lane, level_step_bytes: 128 values (value q of
+// lane j at 32 q + j), then 128 16-bit columns (4 j + q).  Task descriptor: .x log2 G (bits 0-2), R
+// (3-8), S2L_LTASK_* flags, the CTA of an s (12-15), stage (16-31); .y first output slot (0-15),
+// steps (16-31); .z first slot that keeps its right-hand sides; x of block rows: first of bout.
+// Between the two sweeps ybuf holds x by rows, whatever the layouts.
+struct __align__(16) LevelWarp {  // what a warp of a level sweep starts from: one 64-byte load
+    int64_t step, task;  // first step and task
+    int64_t lo;          // offset of the subdomain in the local space
+    int nstep, ntask;
+    int rhs, nrhs;       // its right-hand sides (within the subdomain)
+    int n0;              // single rows without entries: x = right-hand side (slots and right-hand sides 0 .. n0 - 1)
+    int nst;             // stages
+    int T;
+    int pad[3];
+};
+template <typename Real>
+struct LevelFactor {
+    const unsigned char* ent;  // steps; columns are slots: x (< T), the zero slot T, s; values: of single rows
+                               // times 1/diag, of block rows as they are, and the entries of W^-1
+    const Real* dinv;          // per right-hand side in reading order (local space layout): its factor
+    const uint16_t* rslot;     //   and the slot that keeps it
+    const uint4* task;
+    const LevelWarp* warp;     // per (subdomain, CTA, warp)
+    const uint16_t* bout;      // output slots of the tasks of block rows
+    const uint16_t* pos;       // row (local space layout) -> slot of x
+};
+__host__ __device__ constexpr int level_step_bytes(size_t real_bytes) { return (int)(128 * (real_bytes + 2)); }
+
 template <typename Real>
 struct LocalSolveArgs {
+    LevelFactor<Real> lf[2];   // level sweeps (cs > 0), else the dataflow sweeps of f
+    int cs;                    // CTAs per subdomain of the level sweeps
+    int slots;                 // their slots of x and s
     const DevSub* subs;
     const int32_t* sub_list;   // CTA b of a sweep works on subdomain sub_list[b] (nullptr: b)
     SweepFactor<Real> f[2];    // 0 = L (forward), 1 = U (backward)
@@ -223,6 +263,25 @@ void launch_bicg_x(cudaStream_t st, int64_t n, double* x, const double* y, const
                    double omega, double* r, const double* s, const double* t, const double* rh, double* partials,
                    double* out);
 
+// Shared memory of a CTA of the level sweeps: per warp a ring of `depth` steps, and kc columns of
+// `slots` values
+inline size_t level_smem_bytes(size_t real_bytes, int slots, int kc, int depth)
+{
+    return (size_t)(S2L_BS_LEVEL / 32) * depth * level_step_bytes(real_bytes) + (size_t)slots * kc * real_bytes;
+}
+// the deepest ring (8, 4, 3 or 2 steps) that fits
+inline int level_ring(size_t real_bytes, int slots, int kc)
+{
+    for (int depth : {8, 4, 3})
+        if (level_smem_bytes(real_bytes, slots, kc, depth) <= S2L_SWEEP_SMEM_CAP) return depth;
+    return 2;
+}
+// one level sweep of nblocks subdomains, a.K / a.KC clusters each (level_sweep.cu)
+template <typename Real>
+cudaError_t launch_level_sweep(cudaStream_t st, const LocalSolveArgs<Real>& a, bool forward, int nblocks);
+// clusters of cs CTAs with `slots` values each that the device runs at once
+int level_sweep_clusters(size_t real_bytes, int slots, int cs);
+
 // The local solve of every subdomain (or one): forward sweep, tail coupling, two dense tail GEMVs,
 // backward coupling, backward sweep + epilogue.  `tr_range`/`us_range` restrict the row-list
 // kernels (first, count); `launches` receives the number of kernels issued.
@@ -295,6 +354,14 @@ void launch_refactor_blocks(cudaStream_t st, int64_t nblocks, const int64_t* bof
                             const int64_t* wsrc, const int64_t* be_off, const int64_t* be_pos, const uint8_t* be_row,
                             const int64_t* be_cp, const uint8_t* bc_b, const int64_t* bc_pos, const double* F,
                             Real* binv, Real* val);
+// level sweeps: their values, and the dense inverses of their diagonal blocks
+template <typename Real>
+void launch_refactor_level_values(cudaStream_t st, int nwarps, int warps_per_sub, const int64_t* fbase, const double* F,
+                                  const LevelFactor<Real>& lf, const int32_t* src, const int32_t* dsrc,
+                                  unsigned char* ent);
+template <typename Real>
+void launch_refactor_level_blocks(cudaStream_t st, int64_t nblocks, const int32_t* bk, const int64_t* boff,
+                                  const int64_t* wsrc, const int64_t* wpos, const double* F, unsigned char* ent);
 template <typename Real>
 void launch_gather_values(cudaStream_t st, int64_t count, const int64_t* src, const double* F, Real* out);
 void launch_row_sums(cudaStream_t st, int64_t n, const int32_t* rp, const double* v, double* out);

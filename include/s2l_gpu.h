@@ -182,8 +182,13 @@ int s2l_gpu_set_coarse(s2l_setup* s, int64_t n0, const int64_t* offsets, const d
  * chosen per subdomain to minimise 2 * hop_us * (sparse dependency levels) + bytes * nsub / bw_gbs.
  *   "tail_min" (rows, default 64), "tail_max" (default 4096): bounds of a non-empty tail;
  *   "tail_rows" (default 0 = cost model): force every subdomain's tail to this many rows;
- *   "hop_us" (default 0.25), "bw_gbs" (default 6000): the cost model's parameters;
- *   "sweep_group" (0 = 16, 8, 16 or 32): most lanes a sparse-sweep row gets (rows of up to
+ *   "hop_us" (default: 0.25 for dataflow sweeps, 2 for level sweeps), "bw_gbs" (default 6000): the
+ *   cost model's parameters;
+ *   "level_sweeps" (default -1): the sparse sweeps go level by level with a thread-block cluster per
+ *   subdomain and barriers (1: wherever x fits the shared memory), or row by row behind ready flags,
+ *   one CTA per subdomain (0: dataflow sweeps); -1 chooses by the number of dependency levels.
+ *   "chain_block" 1 and AMG local solvers always mean dataflow sweeps;
+ *   "sweep_group" (0 = 16, in level sweeps 32; 8, 16 or 32): most lanes a sparse-sweep row gets (rows of up to
  *   sweep_epl G entries get G lanes, 32 / G rows of one dependency level share a warp);
  *   "sweep_epl" (2, 4, 8 or 16, default 4): entries per lane a sparse-sweep row is sized for (a
  *   row of len entries gets the fewest lanes G, a power of two up to sweep_group, with
@@ -198,21 +203,25 @@ int s2l_gpu_set_coarse(s2l_setup* s, int64_t n0, const int64_t* offsets, const d
  *   "chain_block" (1..16, default 8; 1 = off): rows of a chain block.  Runs of sparse rows where
  *   each row depends on the one solved just before it (the rows of a supernode) are cut into
  *   blocks of up to this many rows; a block's rows are stored multiplied by the inverse of its
- *   diagonal block, so the block is one dependency level of the sweep instead of one per row;
+ *   diagonal block, so the block is one dependency level of the sweep instead of one per row.
+ *   Level sweeps take blocks of up to 8 * chain_block (at most 64) rows and apply the inverse of the
+ *   diagonal block in a step of its own;
  *   "refactor" (0 or 1, default 0): keep the factor patterns and their maps to the solve layout
  *   on the device so s2l_gpu_refactor can refactorize for new matrix values;
  *   "pivot_tol" (default 1e-6, 0 = no check): s2l_gpu_refactor of LU (and LDL^T) factors keeps
  *   the setup's pivot order, and reports S2L_ERR_NUMERIC when a pivot has become small against the
  *   entries it divides (a multiplier larger than 1 / pivot_tol);
  *   "spin_limit" (default 2^24): polls of one ready flag after which a sparse sweep gives up and
- *   the call returns S2L_ERR_TIMEOUT (every wait of the sweeps is bounded).  Unlike the options
+ *   the call returns S2L_ERR_TIMEOUT (every wait of the sweeps is bounded; level sweeps poll
+ *   nothing).  Unlike the options
  *   above it may also be set after s2l_gpu_setup_end; it applies to the launches that follow and
  *   must not be changed while a solve-phase call runs on the setup;
  *   "spin_sleep_ns" (default 0, at most 1e6): a sparse-sweep warp whose poll found a column not
  *   ready pauses this long (__nanosleep) before the next poll, leaving the issue slots to the warps
  *   that compute the rows it waits for.  Like "spin_limit" it may be set after s2l_gpu_setup_end;
  *   "sweep_prefetch" (default 8, 0 to 32): chunks of 32 entries after its current task that a
- *   sparse-sweep warp hints into L2; may be set after s2l_gpu_setup_end.
+ *   sparse-sweep warp hints into L2 (in level sweeps: steps of 128 entries after its ring); may be
+ *   set after s2l_gpu_setup_end.
  */
 int s2l_gpu_setup_option(s2l_setup* s, const char* name, double value);
 
@@ -244,7 +253,8 @@ int s2l_gpu_refactor(s2l_setup* s, const double* val, int ptr_kind);
 /* Device bytes held by the setup (matrix, factors, basis, schedules) and its workspaces. */
 int s2l_gpu_setup_bytes(const s2l_setup* s, size_t* bytes);
 /* Layout statistics after setup_end: "sparse_nnz", "coupling_nnz", "dense_entries", "tail_rows",
-   "sweep_group", "smem_bytes", "levels_max" / "levels_mean" (dependency levels of a sparse sweep,
+   "sweep_group", "smem_bytes", "level_sweeps" (CTAs per subdomain of the level sweeps; 0: dataflow
+   sweeps), "levels_max" / "levels_mean" (dependency levels of a sparse sweep,
    largest and mean over subdomains and both factors), "chain_blocks", "sweep_tasks" and
    "sweep_padding" (padding entries of the lane-interleaved task layout), both factors;
    "local_solve_column_bytes": the part of s2l_gpu_local_solve_bytes that each further right-hand
