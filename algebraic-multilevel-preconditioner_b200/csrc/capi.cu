@@ -203,15 +203,15 @@ struct s2l_setup {
     int nlay = 0;
     void* d_val[2] = {nullptr, nullptr};
     void* d_dinv[2] = {nullptr, nullptr};
-    int32_t *d_tr_sub = nullptr, *d_tr_i = nullptr, *d_lts_col = nullptr;
-    int64_t* d_lts_ptr = nullptr;
-    void* d_lts_val = nullptr;
-    int32_t *d_us_sub = nullptr, *d_us_r = nullptr, *d_ust_col = nullptr, *d_uu = nullptr;
-    int64_t* d_ust_ptr = nullptr;
-    void* d_ust_val = nullptr;
+    int32_t *d_tr_sub = nullptr, *d_tr_i = nullptr;
+    // couplings of the tail rows with the sparse rows (0: L, 1: U)
+    CouplingUnit* d_cu[2] = {nullptr, nullptr};
+    int32_t* d_crow[2] = {nullptr, nullptr};
+    void *d_ccol[2] = {nullptr, nullptr}, *d_cval[2] = {nullptr, nullptr};
+    int cp_wide = 0;
     void *d_linv = nullptr, *d_uinv = nullptr;
     bool need_gflags = false;
-    std::vector<int> tr_first_h, us_first_h, uu_first_h;  // per subdomain, nsub+1 entries
+    std::vector<int> tr_first_h, cu_first_h[2];  // per subdomain, nsub+1 entries
     int sweep_group = 32;
     // options (s2l_gpu_setup_option)
     int opt_tail_min = 64, opt_tail_max = 4096, opt_group = 0, opt_tail_rows = 0, opt_chain = S2L_CHAIN_DEFAULT, opt_block_width = 0,
@@ -287,7 +287,7 @@ struct s2l_setup {
     int opt_refactor = 0;
     struct Refac {
         bool on = false;
-        int64_t nF = 0, nfill = 0, ntc = 0, nlts = 0, nust = 0, nblk[2] = {0, 0};
+        int64_t nF = 0, nfill = 0, ntc = 0, ncsrc[2] = {0, 0}, nblk[2] = {0, 0};
         double* F = nullptr;
         double* S = nullptr;      // dense tails (FP64)
         double* stage = nullptr;  // the new matrix values until they are committed
@@ -299,7 +299,7 @@ struct s2l_setup {
         int32_t *fri = nullptr, *fdg = nullptr, *frpos = nullptr, *frk = nullptr, *lv_first = nullptr,
                 *lv_col = nullptr, *tc_sub = nullptr, *tc_col = nullptr;
         uint8_t* fllt = nullptr;
-        int64_t *fill_src = nullptr, *fill_dst = nullptr, *lts_src = nullptr, *ust_src = nullptr;
+        int64_t *fill_src = nullptr, *fill_dst = nullptr, *csrc[2] = {nullptr, nullptr};
         int32_t *sw_src[2] = {nullptr, nullptr}, *sw_dsrc[2] = {nullptr, nullptr};
         int64_t *wsrc[2] = {nullptr, nullptr}, *be_off[2] = {nullptr, nullptr}, *be_pos[2] = {nullptr, nullptr},
                 *be_cp[2] = {nullptr, nullptr}, *bc_pos[2] = {nullptr, nullptr};
@@ -836,15 +836,6 @@ void build_sweep(const HostCsr& M, int T, bool lower, bool unit_diag, int nw, in
 // smaller rows only) and bytes what one local solve reads for this split: sparse entries of L and
 // U, coupling entries L(T:n, 0:T) and U(0:T, T:n), and the two dense triangles of the tail.  The
 // tail is at most tail_max rows; the sweep's shared memory must hold T rows.  *levels: those of T.
-// Lanes of the U-coupling kernel for a row of `len` entries: about four entries per lane, a power
-// of two, 1 to 32 (a warp takes 32 / lanes rows of about that length)
-int coupling_lanes(int len)
-{
-    int g = 1;
-    while (g < 32 && 4 * g < len) g <<= 1;
-    return g;
-}
-
 int choose_tail(const HostCsr& L, const HostCsr& U, int n, const s2l_tail_model& tm, int* levels)
 {
     // forward levels of L after chain blocking, and the entries blocking adds to each row
@@ -924,6 +915,69 @@ int choose_tail(const HostCsr& L, const HostCsr& U, int n, const s2l_tail_model&
     *levels = maxlev[bestT];
     return bestT;
 }
+
+// The units of one coupling (CouplingUnit), subdomain by subdomain
+struct CouplingList {
+    size_t real_bytes = 8;
+    int per_lane = 16;  // entries a lane takes of a row, at least, before the row gets more lanes
+    std::vector<CouplingUnit> unit;
+    std::vector<int32_t> row, col;
+    std::vector<double> val;
+    std::vector<int64_t> src;  // refactorization: sources of the values (-1: padding)
+    int64_t real = 0;
+
+    // rows (entries, row); entries(row, emit): emit(column, value, source) for each.  Rows that fill a warp keep
+    // their order, the last (longest) first: neighbours read much the same columns, at the same time.  The
+    // others are sorted by length, so a unit's rows are alike.
+    template <typename F>
+    void add(int sub, std::vector<std::pair<int, int>>& rows, bool track, F&& entries)
+    {
+        std::reverse(rows.begin(), rows.end());
+        const auto rest = std::stable_partition(rows.begin(), rows.end(),
+                                                [&](const std::pair<int, int>& x) { return x.first >= 32 * per_lane; });
+        std::stable_sort(rest, rows.end(), [](const std::pair<int, int>& x, const std::pair<int, int>& y) {
+            return x.first > y.first;
+        });
+        for (size_t k = 0; k < rows.size();) {
+            const int len = rows[k].first;
+            int lg = 0;
+            while (lg < 5 && (int64_t)per_lane << (lg + 1) <= len) ++lg;
+            size_t n = std::min(rows.size() - k, (size_t)(32 >> lg));
+            // (rows without entries are units of their own: a padding entry repeats a column of its row)
+            while (len > 0 && rows[k + n - 1].first == 0) --n;
+            const int G = 1 << lg, steps = (len + 4 * G - 1) / (4 * G);
+            const size_t s0 = val.size() / 128;
+            unit.push_back(CouplingUnit{(uint32_t)s0, (int32_t)row.size(), sub, (uint32_t)steps << 9 | (uint32_t)lg << 6 | (uint32_t)n});
+            val.resize(val.size() + (size_t)steps * 128, 0.0);
+            col.resize(val.size(), 0);
+            if (track) src.resize(val.size(), -1);
+            for (size_t i = 0; i < n; ++i) {
+                row.push_back(rows[k + i].second);
+                int e = 0;
+                int32_t last = 0;
+                auto at = [&](int idx, size_t& c, size_t& v) {
+                    const int lane = (int)i * G + idx % G, q = idx / G % 4;
+                    const size_t s = (s0 + (size_t)(idx / (4 * G))) * 128;
+                    c = s + 4 * lane + q;
+                    v = s + coupling_value_pos(real_bytes, lane, q);
+                };
+                size_t c = 0, v = 0;
+                entries(rows[k + i].second, [&](int32_t cc, double vv, int64_t ss) {
+                    at(e++, c, v);
+                    col[c] = last = cc;
+                    val[v] = vv;
+                    if (track) src[v] = ss;
+                    ++real;
+                });
+                for (; e < 4 * G * steps; ++e) {
+                    at(e, c, v);
+                    col[c] = last;
+                }
+            }
+            k += n;
+        }
+    }
+};
 
 // Combined column pattern of one subdomain's factors (RefactorArgs): L L^T the columns of L, LU and
 // LDL^T the strict upper rows (from U), the diagonal (U's), then the strict lower rows (from L).
@@ -1400,15 +1454,8 @@ LocalSolveArgs<Real> solve_args(s2l_work* w, int K, int mode)
     }
     a.tr_sub = s->d_tr_sub;
     a.tr_i = s->d_tr_i;
-    a.lts_ptr = s->d_lts_ptr;
-    a.lts_col = s->d_lts_col;
-    a.lts_val = (const Real*)s->d_lts_val;
-    a.us_sub = s->d_us_sub;
-    a.us_r = s->d_us_r;
-    a.ust_ptr = s->d_ust_ptr;
-    a.ust_col = s->d_ust_col;
-    a.ust_val = (const Real*)s->d_ust_val;
-    a.uu = s->d_uu;
+    for (int f = 0; f < 2; ++f)
+        a.cp[f] = Coupling<Real>{s->d_cu[f], s->d_crow[f], s->d_ccol[f], (const Real*)s->d_cval[f], s->cp_wide};
     a.linv = (const Real*)s->d_linv;
     a.uinv = (const Real*)s->d_uinv;
     a.ylocal = w->d_ylocal;
@@ -1487,6 +1534,18 @@ int amg_local_solve(s2l_work* w, const double* in, const double* base, double* o
                              : amg_local_solve_t<double>(w, in, base, out, mode, only_sub, local_in);
 }
 
+// the tail rows and the units of the couplings (first, count) of one subdomain, or of all (-1)
+void row_ranges(const s2l_setup* s, int sub, int (&tr)[2], int (&cu)[2][2])
+{
+    const int a = std::max(sub, 0), b = sub < 0 ? s->nsub : sub + 1;
+    auto range = [&](const std::vector<int>& first, int (&r)[2]) {
+        r[0] = first[a];
+        r[1] = first[b] - first[a];
+    };
+    range(s->tr_first_h, tr);
+    for (int f = 0; f < 2; ++f) range(s->cu_first_h[f], cu[f]);
+}
+
 int run_local_solve(s2l_work* w, const double* in, const double* base, double* out, int mode, int only_sub,
                     const double* local_in)
 {
@@ -1495,15 +1554,12 @@ int run_local_solve(s2l_work* w, const double* in, const double* base, double* o
     if (s->amgd.on) return amg_local_solve(w, in, base, out, mode, only_sub, local_in);
     const int nb = only_sub >= 0 ? 1 : s->nsub;
     int32_t* sub_list = nullptr;
-    int tr0 = 0, trn = s->tr_first_h[s->nsub], us0 = 0, usn = s->uu_first_h[s->nsub];
+    int tr[2], cu[2][2];
+    row_ranges(s, only_sub, tr, cu);
     if (only_sub >= 0) {
         sub_list = reinterpret_cast<int32_t*>(w->d_red + 500);  // scratch slot for one index
         int32_t v = only_sub;
         CUDA_OK(w, cudaMemcpyAsync(sub_list, &v, sizeof(v), cudaMemcpyHostToDevice, w->stream));
-        tr0 = s->tr_first_h[only_sub];
-        trn = s->tr_first_h[only_sub + 1] - tr0;
-        us0 = s->uu_first_h[only_sub];
-        usn = s->uu_first_h[only_sub + 1] - us0;
     }
     cudaError_t e;
     int launched = 0;
@@ -1515,7 +1571,7 @@ int run_local_solve(s2l_work* w, const double* in, const double* base, double* o
         a.base = base;
         a.out = out;
         a.mode = mode;
-        e = launch_local_solve<float>(w->stream, a, nb, smem, tr0, trn, us0, usn, &launched);
+        e = launch_local_solve<float>(w->stream, a, nb, smem, tr, cu, &launched);
     } else {
         LocalSolveArgs<double> a = solve_args<double>(w, 1, mode);
         a.sub_list = sub_list;
@@ -1523,7 +1579,7 @@ int run_local_solve(s2l_work* w, const double* in, const double* base, double* o
         a.base = base;
         a.out = out;
         a.mode = mode;
-        e = launch_local_solve<double>(w->stream, a, nb, smem, tr0, trn, us0, usn, &launched);
+        e = launch_local_solve<double>(w->stream, a, nb, smem, tr, cu, &launched);
     }
     w->launches += launched;
     if (e != cudaSuccess) return w->fail(S2L_ERR_CUDA, std::string("local_solve launch: ") + cudaGetErrorString(e));
@@ -1680,8 +1736,9 @@ int local_solve_block_t(s2l_work* w, int K, const double* in, const double* base
     if (B.gflags) a.KC = 1;
     const size_t smem = B.gflags ? 0 : sweep_smem(s, a.KC);
     int launched = 0;
-    const cudaError_t e = launch_local_solve<Real>(w->stream, a, s->nsub, smem, 0, s->tr_first_h[s->nsub], 0,
-                                                   s->uu_first_h[s->nsub], &launched);
+    int tr[2], cu[2][2];
+    row_ranges(s, -1, tr, cu);
+    const cudaError_t e = launch_local_solve<Real>(w->stream, a, s->nsub, smem, tr, cu, &launched);
     w->launches += launched;
     if (e != cudaSuccess) return w->fail(S2L_ERR_CUDA, std::string("block local_solve launch: ") + cudaGetErrorString(e));
     return S2L_OK;
@@ -2751,21 +2808,34 @@ int s2l_gpu_setup_end(s2l_setup* s)
     std::vector<int32_t> sw_bfirst[2], sw_bslot[2];
     std::vector<int64_t> sw_boff[2] = {{0}, {0}}, sw_bioff[2] = {{0}, {0}};
     std::vector<double> sw_binv[2];
-    std::vector<int32_t> tr_sub, tr_i, lts_col, us_sub, us_r, ust_col, uu;
-    std::vector<int64_t> lts_ptr(1, 0), ust_ptr(1, 0);
-    std::vector<double> lts_val, ust_val;
+    std::vector<int32_t> tr_sub, tr_i;
+    CouplingList cpl[2];
+    {
+        int64_t cnt = 0;  // entries of U(0:T, T:n), as many as those of L(T:n, 0:T) or about
+        for (int i = 0; i < nsub; ++i)
+            for (int r = 0; r < (s->hs[i].amg ? 0 : Ts[i]); ++r)
+                for (int64_t e = Us[i].rp[r]; e < Us[i].rp[r + 1]; ++e) cnt += Us[i].ci[e] >= Ts[i];
+        // Entries a lane takes of a row: few where the rows are few, for warps and short chains; more where a
+        // warp has many steps to do anyway, for less padding and fewer units.  Local solves in us with 2, 4, 16
+        // and 32: poisson2d 200^2 / 8 (0.3 steps a warp slot) 114, 117, 124, 135; bubbles3d 48^3 / 8 (10 steps)
+        // -, 280, 275, 293; 100^3 / 64 (109 steps) -, 1026, 1003, 997.
+        const double steps = (double)cnt / (128.0 * 32.0 * S2L_SMS);
+        for (auto& c : cpl) {
+            c.real_bytes = rs;
+            c.per_lane = steps >= 32.0 ? 32 : steps >= 4.0 ? 16 : 2;
+        }
+    }
     std::vector<std::vector<double>> Ltt(nsub), Utt(nsub);
     std::vector<int64_t> d_off(nsub + 1, 0);
     s->tr_first_h.assign(nsub + 1, 0);
-    s->us_first_h.assign(nsub + 1, 0);
-    s->uu_first_h.assign(nsub + 1, 0);
+    for (auto& c : s->cu_first_h) c.assign(nsub + 1, 0);
     double bytes = 0.0;
     int max_T = 0, max_nl = 0;
     for (int i = 0; i < nsub; ++i) max_T = std::max(max_T, Ts[i]);
     int64_t sparse_nnz = 0;
     // refactorization plan (host side; see RefactorArgs)
     const bool rfon = s->opt_refactor != 0;
-    std::vector<int64_t> rf_fbase(1, 0), rf_fcp, rf_frp(1, 0), rf_lvoff(1, 0), rf_fill_src, rf_fill_dst, rf_lts, rf_ust;
+    std::vector<int64_t> rf_fbase(1, 0), rf_fcp, rf_frp(1, 0), rf_lvoff(1, 0), rf_fill_src, rf_fill_dst;
     std::vector<int32_t> rf_fri, rf_fdg, rf_frpos, rf_frk, rf_lvfirst, rf_lvcol, rf_tcsub, rf_tccol;
     std::vector<uint8_t> rf_fllt;
     std::vector<int32_t> rf_swsrc[2], rf_swdsrc[2];
@@ -2849,8 +2919,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
         if (pre[i].code != S2L_OK) return s->fail(pre[i].code, "subdomain " + std::to_string(i) + ": " + pre[i].err);
         if (h.amg) {  // AMG local solver: the local space in natural order, no sweeps or tails
             s->tr_first_h[i] = (int)tr_sub.size();
-            s->us_first_h[i] = (int)us_sub.size();
-            s->uu_first_h[i] = (int)uu.size();
+            for (int f = 0; f < 2; ++f) s->cu_first_h[f][i] = (int)cpl[f].unit.size();
             d_off[i + 1] = d_off[i];
             DevSub d{};
             d.begin = h.begin;
@@ -2859,7 +2928,6 @@ int s2l_gpu_setup_end(s2l_setup* s)
             d.n_local = nl;
             d.T = nl;
             d.tr_first = s->tr_first_h[i];
-            d.us_first = s->us_first_h[i];
             d.d_off = d_off[i];
             d.m = h.m;
             d.v_rows = boolean ? h.n_owned : nl;
@@ -3037,17 +3105,17 @@ int s2l_gpu_setup_end(s2l_setup* s)
         }
         // L coupling of the tail rows (columns as forward slots) and the dense lower tail
         s->tr_first_h[i] = (int)tr_sub.size();
+        std::vector<std::pair<int, int>> tlen(sz);  // (coupling entries, tail row)
         if (sz > 0) {
             Ltt[i].assign((size_t)sz * sz, 0.0);
             for (int k = T; k < nl; ++k) {
+                tlen[k - T] = {0, k - T};
                 tr_sub.push_back(i);
                 tr_i.push_back(k - T);
                 for (int64_t e = h.L.rp[k]; e < h.L.rp[k + 1]; ++e) {
                     const int c = h.L.ci[e];
                     if (c < T) {
-                        lts_col.push_back(level ? c : sl.pos[c]);
-                        lts_val.push_back(h.L.v[e]);
-                        if (rfon) rf_lts.push_back(fb + P.find(k, c));
+                        ++tlen[k - T].first;
                     } else if (c < k) {
                         Ltt[i][(size_t)(k - T) * sz + (c - T)] = h.L.v[e];
                     } else if (c == k) {
@@ -3055,7 +3123,6 @@ int s2l_gpu_setup_end(s2l_setup* s)
                     }
                 }
                 if (unitL) Ltt[i][(size_t)(k - T) * sz + (k - T)] = 1.0;
-                lts_ptr.push_back((int64_t)lts_col.size());
             }
             Utt[i].assign((size_t)sz * sz, 0.0);
             for (int k = T; k < nl; ++k)
@@ -3067,38 +3134,29 @@ int s2l_gpu_setup_end(s2l_setup* s)
                 if (Utt[i][(size_t)k * sz + k] == 0.0 || Ltt[i][(size_t)k * sz + k] == 0.0)
                     return s->fail(S2L_ERR_NUMERIC, "subdomain " + std::to_string(i) + ": zero pivot in the dense tail");
         }
-        // U coupling of the sparse rows: the target is the row's forward slot (ybuf keeps forward order).
-        // The rows are stored longest first and grouped into units of one warp: a unit holds rows of
-        // about the same length, each taken by the lanes its length needs (coupling_lanes)
-        s->us_first_h[i] = (int)us_sub.size();
-        s->uu_first_h[i] = (int)uu.size();
+        // the couplings; the sparse rows' columns and targets are forward slots
+        // (level sweeps: rows; ybuf keeps that order)
+        for (int f = 0; f < 2; ++f) s->cu_first_h[f][i] = (int)cpl[f].unit.size();
         if (sz > 0) {
-            std::vector<std::pair<int, int>> rows;  // (tail entries, row)
+            cpl[0].add(i, tlen, rfon, [&](int k, auto emit) {
+                for (int64_t e = h.L.rp[T + k]; e < h.L.rp[T + k + 1]; ++e)
+                    if (const int c = h.L.ci[e]; c < T)
+                        emit(level ? c : sl.pos[c], h.L.v[e], rfon ? fb + P.find(T + k, c) : 0);
+            });
+            std::vector<std::pair<int, int>> rows;  // (tail entries, row as stored)
+            std::vector<int32_t> stored(level ? 0 : T);
             for (int r = 0; r < T; ++r) {
                 int cnt = 0;
                 for (int64_t e = U.rp[r]; e < U.rp[r + 1]; ++e) cnt += U.ci[e] >= T;
-                if (cnt) rows.emplace_back(cnt, r);
+                if (cnt) rows.emplace_back(cnt, level ? r : sl.pos[r]);
+                if (!level) stored[sl.pos[r]] = r;
             }
-            std::stable_sort(rows.begin(), rows.end(), [](const std::pair<int, int>& x, const std::pair<int, int>& y) {
-                return x.first > y.first;
-            });
-            const int q0 = (int)us_sub.size();
-            for (const auto& pr : rows) {
-                const int r = pr.second;
+            cpl[1].add(i, rows, rfon, [&](int q, auto emit) {
+                const int r = level ? q : stored[q];
                 for (int64_t e = U.rp[r]; e < U.rp[r + 1]; ++e)
-                    if (U.ci[e] >= T) {
-                        ust_col.push_back((int32_t)(loc + U.ci[e]));  // local-space index of the tail row
-                        ust_val.push_back(U.v[e]);
-                        if (rfon) rf_ust.push_back(fb + (llt ? P.find(U.ci[e], r) : P.find(r, U.ci[e])));
-                    }
-                us_sub.push_back(i);
-                us_r.push_back(level ? r : sl.pos[r]);
-                ust_ptr.push_back((int64_t)ust_col.size());
-            }
-            for (size_t k = 0; k < rows.size();) {
-                uu.push_back(q0 + (int)k);
-                k += std::min(rows.size() - k, (size_t)(32 / coupling_lanes(rows[k].first)));
-            }
+                    if (U.ci[e] >= T)
+                        emit(U.ci[e] - T, U.v[e], rfon ? fb + (llt ? P.find(U.ci[e], r) : P.find(r, U.ci[e])) : 0);
+            });
         }
         d_off[i + 1] = d_off[i] + (int64_t)sz * sz;
         DevSub d{};
@@ -3108,7 +3166,6 @@ int s2l_gpu_setup_end(s2l_setup* s)
         d.n_local = nl;
         d.T = T;
         d.tr_first = s->tr_first_h[i];
-        d.us_first = s->us_first_h[i];
         d.d_off = d_off[i];
         d.m = h.m;
         d.v_rows = boolean ? h.n_owned : nl;
@@ -3136,15 +3193,15 @@ int s2l_gpu_setup_end(s2l_setup* s)
         Us[i] = HostCsr();
     }
     s->tr_first_h[nsub] = (int)tr_sub.size();
-    s->us_first_h[nsub] = (int)us_sub.size();
-    s->uu_first_h[nsub] = (int)uu.size();
-    uu.push_back((int32_t)us_sub.size());  // the end of the last unit
+    for (int f = 0; f < 2; ++f) s->cu_first_h[f][nsub] = (int)cpl[f].unit.size();
+    s->cp_wide = max_nl > 65536;
     s->nloc = loc;
     if (!level) s->st_sparse_nnz = sparse_nnz;
-    s->st_coupling_nnz = (int64_t)lts_col.size() + (int64_t)ust_col.size();
+    s->st_coupling_nnz = cpl[0].real + cpl[1].real;
     s->st_dense_entries = d_off[nsub];
     s->st_tail_rows = (int64_t)tr_sub.size();
-    bytes += (double)s->st_coupling_nnz * (rs + 4) + (double)(tr_sub.size() + us_sub.size()) * (8 + 8 + rs);
+    bytes += (double)s->st_coupling_nnz * (rs + (s->cp_wide ? 4 : 2));
+    for (const auto& c : cpl) bytes += (double)c.row.size() * (4 + 2 * rs) + (double)c.unit.size() * sizeof(CouplingUnit);
     if (level) bytes += s->solve_bytes;  // (the sparse parts of build_level_layouts)
     for (int f = 0; f < 2 && !level; ++f) {
         sw_wtask[f].push_back((int64_t)sw_thdr[f].size());
@@ -3179,19 +3236,19 @@ int s2l_gpu_setup_end(s2l_setup* s)
     RET_IF(upload(s, &s->d_u2l, u2l));
     RET_IF(upload(s, &s->d_tr_sub, tr_sub));
     RET_IF(upload(s, &s->d_tr_i, tr_i));
-    RET_IF(upload(s, &s->d_lts_ptr, lts_ptr));
-    RET_IF(upload(s, &s->d_lts_col, lts_col));
-    RET_IF(upload(s, &s->d_us_sub, us_sub));
-    RET_IF(upload(s, &s->d_us_r, us_r));
-    RET_IF(upload(s, &s->d_ust_ptr, ust_ptr));
-    RET_IF(upload(s, &s->d_ust_col, ust_col));
-    RET_IF(upload(s, &s->d_uu, uu));
+    for (int f = 0; f < 2; ++f) {
+        RET_IF(upload(s, &s->d_cu[f], cpl[f].unit));
+        RET_IF(upload(s, &s->d_crow[f], cpl[f].row));
+        if (s->cp_wide) {
+            RET_IF(upload(s, (int32_t**)&s->d_ccol[f], cpl[f].col));
+        } else {
+            RET_IF(upload(s, (uint16_t**)&s->d_ccol[f], std::vector<uint16_t>(cpl[f].col.begin(), cpl[f].col.end())));
+        }
+    }
     if (s->real == S2L_REAL_F32) {
-        RET_IF(upload_real<float>(s, &s->d_lts_val, lts_val));
-        RET_IF(upload_real<float>(s, &s->d_ust_val, ust_val));
+        for (int f = 0; f < 2; ++f) RET_IF(upload_real<float>(s, &s->d_cval[f], cpl[f].val));
     } else {
-        RET_IF(upload_real<double>(s, &s->d_lts_val, lts_val));
-        RET_IF(upload_real<double>(s, &s->d_ust_val, ust_val));
+        for (int f = 0; f < 2; ++f) RET_IF(upload_real<double>(s, &s->d_cval[f], cpl[f].val));
     }
     // ---- dense tail inverses on the device (FP64 triangular solves with the identity)
     RET_IF(dev_alloc(s, &s->d_linv, (size_t)std::max<int64_t>(d_off[nsub], 1) * rs));
@@ -3299,8 +3356,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
         R.nF = rf_fbase.back();
         R.nfill = (int64_t)rf_fill_src.size();
         R.ntc = (int64_t)rf_tcsub.size();
-        R.nlts = (int64_t)rf_lts.size();
-        R.nust = (int64_t)rf_ust.size();
+        for (int f = 0; f < 2; ++f) R.ncsrc[f] = (int64_t)cpl[f].src.size();
         R.d_off = d_off;
         RET_IF(dev_alloc(s, reinterpret_cast<void**>(&R.F), (size_t)std::max<int64_t>(R.nF, 1) * sizeof(double)));
         RET_IF(dev_alloc(s, reinterpret_cast<void**>(&R.S), (size_t)std::max<int64_t>(d_off[nsub], 1) * sizeof(double)));
@@ -3444,8 +3500,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
         RET_IF(upload(s, &R.tc_col, rf_tccol));
         RET_IF(upload(s, &R.fill_src, rf_fill_src));
         RET_IF(upload(s, &R.fill_dst, rf_fill_dst));
-        RET_IF(upload(s, &R.lts_src, rf_lts));
-        RET_IF(upload(s, &R.ust_src, rf_ust));
+        for (int f = 0; f < 2; ++f) RET_IF(upload(s, &R.csrc[f], cpl[f].src));
         for (int f = 0; f < 2; ++f) {
             R.nblk[f] = (int64_t)rf_beoff[f].size() - 1;
             RET_IF(upload(s, &R.sw_src[f], rf_swsrc[f]));
@@ -3656,8 +3711,7 @@ int refactor_commit_factors(s2l_setup* s, cudaStream_t st)
                                      R.be_row[f], R.be_cp[f], R.bc_b[f], R.bc_pos[f], R.F, (Real*)s->d_binv[f],
                                      (Real*)s->d_val[f]);
     }
-    launch_gather_values<Real>(st, R.nlts, R.lts_src, R.F, (Real*)s->d_lts_val);
-    launch_gather_values<Real>(st, R.nust, R.ust_src, R.F, (Real*)s->d_ust_val);
+    for (int f = 0; f < 2; ++f) launch_gather_values<Real>(st, R.ncsrc[f], R.csrc[f], R.F, (Real*)s->d_cval[f]);
     // dense tail inverses: the triangles of each factored tail inverted (cusolverDnXtrtri), the
     // subdomains spread over the tail streams.  Column-major, the tail holds the Cholesky factor
     // U_c (upper; row-major that is the lower L) or U' (upper) and L' (strict lower, unit diagonal);

@@ -5,6 +5,8 @@
 // fixed order.  The same input therefore gives bitwise-identical results, alone or in a batch.
 #include "s2l_internal.cuh"
 
+#include <type_traits>
+
 namespace s2l {
 
 namespace {
@@ -579,62 +581,6 @@ __device__ __forceinline__ void load_k(const Real* __restrict__ p, Real (&v)[K])
     }
 }
 
-// acc[r] = sum_e val[e] * x[col[e] * K + r] over e in [e0, e1), one warp; for K = 1 four
-// independent gathers are in flight per lane, for K > 1 the K columns give the independence
-template <typename Real, int K>
-__device__ __forceinline__ void warp_gather_dot(const Real* __restrict__ val, const int32_t* __restrict__ col,
-                                                int64_t e0, int64_t e1, const Real* __restrict__ x, int lane,
-                                                Real (&acc)[K])
-{
-    if (K == 1) {
-        Real a0 = Real(0), a1 = Real(0), a2 = Real(0), a3 = Real(0);
-        int64_t e = e0 + lane;
-        for (; e + 96 < e1; e += 128) {
-            const int c0 = col[e], c1 = col[e + 32], c2 = col[e + 64], c3 = col[e + 96];
-            const Real v0 = val[e], v1 = val[e + 32], v2 = val[e + 64], v3 = val[e + 96];
-            a0 += v0 * x[c0];
-            a1 += v1 * x[c1];
-            a2 += v2 * x[c2];
-            a3 += v3 * x[c3];
-        }
-        for (; e < e1; e += 32) a0 += val[e] * x[col[e]];
-        acc[0] = warp_sum((a0 + a1) + (a2 + a3));
-    } else {
-#pragma unroll
-        for (int r = 0; r < K; ++r) acc[r] = Real(0);
-        int64_t e = e0 + lane;
-        for (; e + 96 < e1; e += 128) {  // four entries in flight per lane
-            const int c0 = col[e], c1 = col[e + 32], c2 = col[e + 64], c3 = col[e + 96];
-            const Real v0 = val[e], v1 = val[e + 32], v2 = val[e + 64], v3 = val[e + 96];
-            Real x0[K], x1[K], x2[K], x3[K];
-            load_k<Real, K>(x + (int64_t)c0 * K, x0);
-            load_k<Real, K>(x + (int64_t)c1 * K, x1);
-            load_k<Real, K>(x + (int64_t)c2 * K, x2);
-            load_k<Real, K>(x + (int64_t)c3 * K, x3);
-#pragma unroll
-            for (int r = 0; r < K; ++r) acc[r] += (v0 * x0[r] + v1 * x1[r]) + (v2 * x2[r] + v3 * x3[r]);
-        }
-        for (; e + 32 < e1; e += 64) {
-            const int c0 = col[e], c1 = col[e + 32];
-            const Real v0 = val[e], v1 = val[e + 32];
-            Real x0[K], x1[K];
-            load_k<Real, K>(x + (int64_t)c0 * K, x0);
-            load_k<Real, K>(x + (int64_t)c1 * K, x1);
-#pragma unroll
-            for (int r = 0; r < K; ++r) acc[r] += v0 * x0[r] + v1 * x1[r];
-        }
-        if (e < e1) {
-            const Real v0 = val[e];
-            Real x0[K];
-            load_k<Real, K>(x + (int64_t)col[e] * K, x0);
-#pragma unroll
-            for (int r = 0; r < K; ++r) acc[r] += v0 * x0[r];
-        }
-#pragma unroll
-        for (int r = 0; r < K; ++r) acc[r] = warp_allsum(acc[r]);  // lane r writes column r
-    }
-}
-
 // lane r < K gets acc[r] (a register array indexed by a runtime lane)
 template <typename Real, int K>
 __device__ __forceinline__ Real pick(const Real (&acc)[K], int lane)
@@ -646,20 +592,172 @@ __device__ __forceinline__ Real pick(const Real (&acc)[K], int lane)
     return mine;
 }
 
-// Tail right-hand side: t(T+i) = b(T+i) - L(T+i, 0:T) y(0:T), one warp per tail row, K columns.
-template <typename Real, int K>
-__global__ void __launch_bounds__(256) tail_rhs_kernel(const LocalSolveArgs<Real> a, int q0, int count)
+// The couplings, K columns.  L: t(T+i) = b(T+i) - L(T+i, 0:T) y(0:T) of the tail rows; U: y(r) -= U(r, T:n)
+// x(T:n) of the sparse rows that have tail columns.  One warp per unit (CouplingUnit).
+//
+// Bound by memory: 16-bit columns relative to the subdomain, one load for a lane's four columns and one or two
+// for its values (10 bytes an entry in FP64, 6 in FP32; 12 and 8 with 32-bit columns and a load each before).
+// Two steps of a unit are in flight; consecutive lanes hold consecutive entries, whose columns mostly lie side by
+// side, so the gathers coalesce.  With more than 16 bytes of x per entry a lane reading all of them would
+// touch every sector several times (16 columns, FP32, bubbles3d 100^3 / 64: 587 us a coupling), so lanes share.
+template <bool ONCE>
+__device__ __forceinline__ uint4 load16(const uint4* p)  // ONCE: past L1, which is left to the gathers
 {
-    const int q = q0 + blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (!ONCE) return __ldg(p);
+    uint4 w;
+    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "l"(p));
+    return w;
+}
+template <bool ONCE>
+__device__ __forceinline__ uint2 load8(const uint2* p)
+{
+    if (!ONCE) return __ldg(p);
+    uint2 w;
+    asm("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(w.x), "=r"(w.y) : "l"(p));
+    return w;
+}
+
+template <typename Real, typename Col>
+struct CouplingStep {
+    Real v[4];
+    Col c[4];
+    template <bool ONCE>
+    __device__ __forceinline__ void load(const Real* val, const Col* col, uint32_t step, int lane)
+    {
+        const uint4* vp = reinterpret_cast<const uint4*>(val + (int64_t)step * 128) + lane;
+        if (sizeof(Real) == 4) {
+            const uint4 w = load16<ONCE>(vp);
+            __builtin_memcpy(v, &w, 16);
+        } else {
+            const uint4 w0 = load16<ONCE>(vp), w1 = load16<ONCE>(vp + 32);
+            __builtin_memcpy(v, &w0, 16);
+            __builtin_memcpy(reinterpret_cast<char*>(v) + 16, &w1, 16);
+        }
+        if (sizeof(Col) == 2) {
+            const uint2 w = load8<ONCE>(reinterpret_cast<const uint2*>(col + (int64_t)step * 128) + lane);
+            __builtin_memcpy(c, &w, 8);
+        } else {
+            const uint4 w = load16<ONCE>(reinterpret_cast<const uint4*>(col + (int64_t)step * 128) + lane);
+            __builtin_memcpy(c, &w, 16);
+        }
+    }
+    template <int K>
+    __device__ __forceinline__ void add(const Real* x, Real (&acc)[K]) const
+    {
+        Real t[4][K];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) load_k<Real, K>(x + (int64_t)c[q] * K, t[q]);
+#pragma unroll
+        for (int r = 0; r < K; ++r) acc[r] += (v[0] * t[0][r] + v[1] * t[1][r]) + (v[2] * t[2][r] + v[3] * t[3][r]);
+    }
+};
+
+template <typename Real, int N>
+struct CouplingSum {
+    Real v[N];
+};
+
+template <typename Real, typename Col, int K, bool TAIL_RHS>
+__global__ void __launch_bounds__(256) coupling_kernel(const LocalSolveArgs<Real> a, int u0, int count)
+{
+    const Coupling<Real>& cf = a.cp[TAIL_RHS ? 0 : 1];
+    const int u = u0 + blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    if (q >= q0 + count) return;
-    const DevSub sd = a.subs[a.tr_sub[q]];
+    if (u >= u0 + count) return;
+    const CouplingUnit cu = cf.unit[u];
+    const int n = cu.nsteps_lg_n & 63, lg = (cu.nsteps_lg_n >> 6) & 7, nsteps = (int)(cu.nsteps_lg_n >> 9);
+    const DevSub sd = a.subs[cu.sub];
     const int64_t lo = sd.loc_off;
-    const int k = sd.T + a.tr_i[q];
-    Real acc[K];
-    warp_gather_dot<Real, K>(a.lts_val, a.lts_col, a.lts_ptr[q], a.lts_ptr[q + 1], a.ybuf + lo * K, lane, acc);
-    if (lane < K)
-        a.ybuf[(lo + k) * K + lane] = (Real)a.in[(int64_t)a.gather[lo + k] * K + lane] - pick<Real, K>(acc, lane);
+    const Real* x = a.ybuf + (TAIL_RHS ? lo : lo + sd.T) * K;
+    const Col* col = (const Col*)cf.col;
+    // this lane's row, where it is, its index into the right-hand side and (one column) the value, ahead of the sum
+    const int ri = lane >> lg;
+    const int row = ri < n ? cf.row[cu.row + ri] : -1;
+    const int64_t k0 = row < 0 ? -1 : lo + (TAIL_RHS ? sd.T + row : row);
+    const int g0 = TAIL_RHS && row >= 0 ? a.gather[k0] : 0;
+    Real b0 = Real(0);
+    if (K == 1 && row >= 0) b0 = TAIL_RHS ? (Real)a.in[g0] : a.ybuf[k0];
+    // the right-hand side (L) or the row itself (U), less the sum of columns r and on
+    auto put = [&](int64_t k, int g, int r, auto sum) {
+        if (k < 0) return;
+        const double* in = a.in + (int64_t)g * K + r;
+        Real* y = a.ybuf + k * K + r;
+#pragma unroll
+        for (int q = 0; q < (int)(sizeof(sum.v) / sizeof(Real)); ++q)
+            y[q] = (K == 1 ? b0 : TAIL_RHS ? (Real)in[q] : y[q]) - sum.v[q];
+    };
+    const int G = 1 << lg;
+    constexpr int P = K * (int)sizeof(Real) > 16 ? K * (int)sizeof(Real) / 16 : 1;
+    if constexpr (P == 1) {
+        Real acc[K];
+#pragma unroll
+        for (int r = 0; r < K; ++r) acc[r] = Real(0);
+        CouplingStep<Real, Col> s0, s1;
+        int s = 0;
+#pragma unroll 1
+        for (; s + 1 < nsteps; s += 2) {
+            s0.template load<true>(cf.val, col, cu.step + s, lane);
+            s1.template load<true>(cf.val, col, cu.step + s + 1, lane);
+            s0.template add<K>(x, acc);
+            s1.template add<K>(x, acc);
+        }
+        if (s < nsteps) {
+            s0.template load<true>(cf.val, col, cu.step + s, lane);
+            s0.template add<K>(x, acc);
+        }
+#pragma unroll
+        for (int r = 0; r < K; ++r)
+            for (int o = G >> 1; o; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+#pragma unroll
+        for (int r = 0; r < K; ++r)  // the lanes of a row share its columns out
+            if ((lane & (G - 1)) == (r & (G - 1))) put(k0, g0, r, CouplingSum<Real, 1>{{acc[r]}});
+    } else {
+        // P lanes side by side read the 16-byte parts of one entry's x together, so a gather of 32 / P entries
+        // touches no sector twice; they take the entries of their P lanes one lane after the other
+        constexpr int V = 16 / (int)sizeof(Real);
+        const int part = lane & (P - 1), own = lane & ~(P - 1);
+        Real acc[P][V];
+#pragma unroll
+        for (int o = 0; o < P; ++o)
+#pragma unroll
+            for (int q = 0; q < V; ++q) acc[o][q] = Real(0);
+#pragma unroll 1
+        for (int s = 0; s < nsteps; ++s)
+#pragma unroll
+            for (int o = 0; o < P; ++o) {
+                CouplingStep<Real, Col> e;
+                e.template load<false>(cf.val, col, cu.step + s, own + o);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    Real t[V];
+                    const uint4 w = __ldg(reinterpret_cast<const uint4*>(x + (int64_t)e.c[q] * K) + part);
+                    __builtin_memcpy(t, &w, 16);
+#pragma unroll
+                    for (int r = 0; r < V; ++r) acc[o][r] += e.v[q] * t[r];
+                }
+            }
+        if (G >= P) {  // one row: all of the lane's sums, then those of the row's other lanes
+            CouplingSum<Real, V> sum{};
+#pragma unroll
+            for (int r = 0; r < V; ++r) {
+#pragma unroll
+                for (int o = 0; o < P; ++o) sum.v[r] += acc[o][r];
+                for (int o = G >> 1; o >= P; o >>= 1) sum.v[r] += __shfl_xor_sync(0xffffffffu, sum.v[r], o);
+            }
+            if ((lane & (G - 1)) < P) put(k0, g0, part * V, sum);
+        } else {  // P / G rows
+            CouplingSum<Real, V> sum{};
+#pragma unroll
+            for (int o = 0; o < P; ++o) {
+#pragma unroll
+                for (int r = 0; r < V; ++r) sum.v[r] += acc[o][r];
+                if ((o & (G - 1)) == G - 1) {
+                    put(__shfl_sync(0xffffffffu, k0, own + o), __shfl_sync(0xffffffffu, g0, own + o), part * V, sum);
+                    sum = CouplingSum<Real, V>{};
+                }
+            }
+        }
+    }
 }
 
 // Dense tail: out(T+i) = sum_j Minv(i, j) in(T+j), j <= i (lower) or j >= i (upper); warp per row,
@@ -725,55 +823,6 @@ __global__ void __launch_bounds__(256) tail_gemv_kernel(const LocalSolveArgs<Rea
 #pragma unroll
         for (int r = 0; r < K; ++r) acc[r] = warp_allsum(acc[r]);  // lane r writes column r
         if (lane < K) vout[(base + i) * K + lane] = pick<Real, K>(acc, lane);
-    }
-}
-
-// Backward coupling: y(r) -= U(r, T:n) x(T:n) for the sparse rows that have tail columns, K columns.
-// One warp per unit of rows of about the same length (stored longest first): with n rows in the
-// unit, G = 32 / n lanes (a power of two) take each row, each lane with four entries in flight,
-// and the G partial sums of a row are added by a butterfly within its lane group.
-template <typename Real, int K>
-__global__ void __launch_bounds__(256) sparse_coupling_kernel(const LocalSolveArgs<Real> a, int u0, int ucount)
-{
-    const int u = u0 + blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (u >= u0 + ucount) return;
-    const int qa = a.uu[u], n = a.uu[u + 1] - qa;  // 1 <= n <= 32
-    int lg = 5;
-    while ((n << lg) > 32) --lg;  // G = 2^lg lanes per row, the largest with G n <= 32
-    const int G = 1 << lg, ri = lane >> lg, sl = lane & (G - 1);
-    const bool valid = ri < n;
-    const int q = qa + (valid ? ri : 0);
-    int64_t e = a.ust_ptr[q] + sl;
-    const int64_t e1 = valid ? a.ust_ptr[q + 1] : e;
-    Real acc[K];
-#pragma unroll
-    for (int r = 0; r < K; ++r) acc[r] = Real(0);
-    for (; e + 3 * G < e1; e += 4 * G) {
-        const int c0 = a.ust_col[e], c1 = a.ust_col[e + G], c2 = a.ust_col[e + 2 * G], c3 = a.ust_col[e + 3 * G];
-        const Real v0 = a.ust_val[e], v1 = a.ust_val[e + G], v2 = a.ust_val[e + 2 * G], v3 = a.ust_val[e + 3 * G];
-        Real x0[K], x1[K], x2[K], x3[K];
-        load_k<Real, K>(a.ybuf + (int64_t)c0 * K, x0);
-        load_k<Real, K>(a.ybuf + (int64_t)c1 * K, x1);
-        load_k<Real, K>(a.ybuf + (int64_t)c2 * K, x2);
-        load_k<Real, K>(a.ybuf + (int64_t)c3 * K, x3);
-#pragma unroll
-        for (int r = 0; r < K; ++r) acc[r] += (v0 * x0[r] + v1 * x1[r]) + (v2 * x2[r] + v3 * x3[r]);
-    }
-    for (; e < e1; e += G) {
-        const Real v0 = a.ust_val[e];
-        Real x0[K];
-        load_k<Real, K>(a.ybuf + (int64_t)a.ust_col[e] * K, x0);
-#pragma unroll
-        for (int r = 0; r < K; ++r) acc[r] += v0 * x0[r];
-    }
-#pragma unroll
-    for (int r = 0; r < K; ++r)
-        for (int o = G >> 1; o; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
-    if (valid && sl == 0) {
-        const int64_t o = (a.subs[a.us_sub[q]].loc_off + a.us_r[q]) * K;
-#pragma unroll
-        for (int r = 0; r < K; ++r) a.ybuf[o + r] -= acc[r];
     }
 }
 
@@ -1612,9 +1661,17 @@ void launch_bicg_x(cudaStream_t st, int64_t n, double* x, const double* y, const
 }
 
 template <typename Real, int KC, int K>
-cudaError_t launch_local_solve_k(cudaStream_t st, const LocalSolveArgs<Real>& a, int nblocks, size_t smem, int tr_first,
-                                 int tr_count, int uu_first, int uu_count, int* launches)
+cudaError_t launch_local_solve_k(cudaStream_t st, const LocalSolveArgs<Real>& a, int nblocks, size_t smem,
+                                 const int (&tr)[2], const int (&cu)[2][2], int* launches)
 {
+    auto couple = [&](auto rhs) {
+        constexpr bool RHS = decltype(rhs)::value;
+        const int first = cu[RHS ? 0 : 1][0], count = cu[RHS ? 0 : 1][1];
+        if (count == 0) return 0;
+        if (a.cp[RHS ? 0 : 1].wide) coupling_kernel<Real, int32_t, K, RHS><<<(count + 7) / 8, 256, 0, st>>>(a, first, count);
+        else coupling_kernel<Real, uint16_t, K, RHS><<<(count + 7) / 8, 256, 0, st>>>(a, first, count);
+        return 1;
+    };
     cudaError_t e;
     const int grid = nblocks * (K / KC);
     if (a.cs > 0) {
@@ -1635,17 +1692,14 @@ cudaError_t launch_local_solve_k(cudaStream_t st, const LocalSolveArgs<Real>& a,
         sweep_kernel<Real, false, true, KC><<<grid, S2L_BS_SWEEP, 0, st>>>(a);
     }
     int nl = 1;
-    if (tr_count > 0) {
-        const int g = (tr_count + 7) / 8;
-        tail_rhs_kernel<Real, K><<<g, 256, 0, st>>>(a, tr_first, tr_count);
-        tail_gemv_kernel<Real, true, K><<<g, 256, 0, st>>>(a, a.linv, a.ybuf, a.xbuf, tr_first, tr_count);
-        tail_gemv_kernel<Real, false, K><<<g, 256, 0, st>>>(a, a.uinv, a.xbuf, a.ybuf, tr_first, tr_count);
-        nl += 3;
+    if (tr[1] > 0) {
+        const int g = (tr[1] + 7) / 8;
+        nl += couple(std::true_type{});
+        tail_gemv_kernel<Real, true, K><<<g, 256, 0, st>>>(a, a.linv, a.ybuf, a.xbuf, tr[0], tr[1]);
+        tail_gemv_kernel<Real, false, K><<<g, 256, 0, st>>>(a, a.uinv, a.xbuf, a.ybuf, tr[0], tr[1]);
+        nl += 2;
     }
-    if (uu_count > 0) {
-        sparse_coupling_kernel<Real, K><<<(uu_count + 7) / 8, 256, 0, st>>>(a, uu_first, uu_count);
-        nl += 1;
-    }
+    nl += couple(std::false_type{});
     if (a.cs > 0) {
         e = launch_level_sweep<Real>(st, a, false, nblocks);
         if (e != cudaSuccess) return e;
@@ -1658,15 +1712,14 @@ cudaError_t launch_local_solve_k(cudaStream_t st, const LocalSolveArgs<Real>& a,
 }
 
 template <typename Real>
-cudaError_t launch_local_solve(cudaStream_t st, const LocalSolveArgs<Real>& a, int nblocks, size_t smem, int tr_first,
-                               int tr_count, int uu_first, int uu_count, int* launches)
+cudaError_t launch_local_solve(cudaStream_t st, const LocalSolveArgs<Real>& a, int nblocks, size_t smem,
+                               const int (&tr)[2], const int (&cu)[2][2], int* launches)
 {
     // (KC, K): right-hand sides per sweep CTA and in all; the setup's shared memory fixes KC
     const int K = a.K, KC = a.cs > 0 || smem > 0 ? a.KC : 1;
 #define S2L_LS(KC_, K_)                                                                                         \
     if (KC == KC_ && K == K_)                                                                                  \
-    return launch_local_solve_k<Real, KC_, K_>(st, a, nblocks, smem, tr_first, tr_count, uu_first, uu_count, \
-                                               launches)
+    return launch_local_solve_k<Real, KC_, K_>(st, a, nblocks, smem, tr, cu, launches)
     S2L_LS(1, 1);
     S2L_LS(1, 2);
     S2L_LS(2, 2);
@@ -1683,10 +1736,10 @@ cudaError_t launch_local_solve(cudaStream_t st, const LocalSolveArgs<Real>& a, i
     return cudaErrorInvalidValue;
 }
 
-template cudaError_t launch_local_solve<double>(cudaStream_t, const LocalSolveArgs<double>&, int, size_t, int, int, int,
-                                                int, int*);
-template cudaError_t launch_local_solve<float>(cudaStream_t, const LocalSolveArgs<float>&, int, size_t, int, int, int,
-                                                int, int*);
+template cudaError_t launch_local_solve<double>(cudaStream_t, const LocalSolveArgs<double>&, int, size_t, const int (&)[2],
+                                                const int (&)[2][2], int*);
+template cudaError_t launch_local_solve<float>(cudaStream_t, const LocalSolveArgs<float>&, int, size_t, const int (&)[2],
+                                                const int (&)[2][2], int*);
 
 void launch_to_float(cudaStream_t st, const double* in, float* out, int64_t n)
 {

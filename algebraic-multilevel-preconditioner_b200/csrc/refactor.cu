@@ -540,7 +540,7 @@ __global__ void gather_values_kernel(int64_t count, const int64_t* __restrict__ 
                                      Real* __restrict__ out)
 {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x)
-        out[e] = (Real)F[src[e]];
+        out[e] = src[e] >= 0 ? (Real)F[src[e]] : Real(0);  // (negative: padding)
 }
 
 // A 1 in row order (the same summation order as the host's)

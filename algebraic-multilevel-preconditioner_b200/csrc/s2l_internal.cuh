@@ -35,6 +35,7 @@
 #define S2L_SPIN_SLEEP_NS 0   // pause of a sweep warp after a poll that found a column not ready (ns; 0 = none)
 #endif
 #define S2L_SPIN_LIMIT (1 << 24)  // polls of one ready flag before a sweep gives up (error 1)
+#define S2L_SMS 148           // SMs that rules on sizes count on
 #define S2L_BS_LEVEL 512      // threads of a CTA of the level sweeps (level_sweep.cu)
 #define S2L_LEVEL_HOP_US 2.0  // the tail split's time of a level of a level sweep (hop_us default)
 #define S2L_LEVEL_CAP 64      // rows of a block of the level sweeps, at most
@@ -51,7 +52,6 @@ struct DevSub {
     int n_local;
     int T;              // rows [0, T) sparse, [T, n_local) dense tail
     int tr_first;       // first entry of the subdomain in the tail-row list
-    int us_first;       // first entry of the subdomain in the sparse-row coupling list
     int pad;
     int64_t d_off;      // offset of the subdomain's s x s inverse tails
     // coarse basis
@@ -115,6 +115,30 @@ struct LevelFactor {
 };
 __host__ __device__ constexpr int level_step_bytes(size_t real_bytes) { return (int)(128 * (real_bytes + 2)); }
 
+// Coupling rows between the sparse part and the tail in units of one warp: 2^lg lanes per row, 32 / 2^lg
+// rows of about one length.  A unit's entries are steps of 128, four to a lane: entry e of a row is entry
+// q = e / 2^lg mod 4 of the row's lane e mod 2^lg in the unit's step e / 2^(lg + 2).  A step holds the lanes'
+// columns at 4 lane + q, and their values at coupling_value_pos, so a lane takes its columns with one load
+// and its values with 16-byte loads.
+struct CouplingUnit {
+    uint32_t step;       // first step
+    int32_t row;         // first row in the row list
+    int32_t sub;
+    uint32_t nsteps_lg_n;  // steps << 9 | lg << 6 | rows
+};
+template <typename Real>
+struct Coupling {
+    const CouplingUnit* unit;
+    const int32_t* row;
+    const void* col;     // 16 bits, or 32 where a subdomain has more than 65536 rows
+    const Real* val;
+    int wide;            // 32-bit columns
+};
+__host__ __device__ constexpr int coupling_value_pos(size_t real_bytes, int lane, int q)
+{
+    return real_bytes == 4 ? 4 * lane + q : 64 * (q >> 1) + 2 * lane + (q & 1);
+}
+
 template <typename Real>
 struct LocalSolveArgs {
     LevelFactor<Real> lf[2];   // level sweeps (cs > 0), else the dataflow sweeps of f
@@ -123,21 +147,11 @@ struct LocalSolveArgs {
     const DevSub* subs;
     const int32_t* sub_list;   // CTA b of a sweep works on subdomain sub_list[b] (nullptr: b)
     SweepFactor<Real> f[2];    // 0 = L (forward), 1 = U (backward)
-    // tail rows of every subdomain: (sub, i) pairs, L(T+i, 0:T) coupling CSR
+    // tail rows of every subdomain: (sub, i) pairs
     const int32_t* tr_sub;
     const int32_t* tr_i;
-    const int64_t* lts_ptr;
-    const int32_t* lts_col;
-    const Real* lts_val;
-    // sparse rows with U(r, T:n) coupling: (sub, r) pairs and CSR (columns as local-space indices,
-    // loc_off + tail row), longest rows first within a subdomain; unit u (one warp) holds the rows
-    // uu[u] .. uu[u + 1] - 1, 32 / (its row count) lanes per row
-    const int32_t* us_sub;
-    const int32_t* us_r;
-    const int64_t* ust_ptr;
-    const int32_t* ust_col;
-    const Real* ust_val;
-    const int32_t* uu;
+    // 0: L(T+i, 0:T) (row i, columns: sparse rows), 1: U(r, T:n) (row r, columns: tail rows from 0 on)
+    Coupling<Real> cp[2];
     const Real* linv;          // inverse tails, row-major per subdomain
     const Real* uinv;
     const int32_t* gather;     // slot k -> index into `in` (global gather, or perm_in for a local input)
@@ -283,11 +297,11 @@ cudaError_t launch_level_sweep(cudaStream_t st, const LocalSolveArgs<Real>& a, b
 int level_sweep_clusters(size_t real_bytes, int slots, int cs);
 
 // The local solve of every subdomain (or one): forward sweep, tail coupling, two dense tail GEMVs,
-// backward coupling, backward sweep + epilogue.  `tr_range`/`us_range` restrict the row-list
-// kernels (first, count); `launches` receives the number of kernels issued.
+// backward coupling, backward sweep + epilogue.  tr and cu restrict the row-list kernels (first,
+// count of the tail rows and of the two couplings' units); `launches` receives the number of kernels issued.
 template <typename Real>
 cudaError_t launch_local_solve(cudaStream_t st, const LocalSolveArgs<Real>& a, int nblocks, size_t smem_bytes,
-                               int tr_first, int tr_count, int uu_first, int uu_count, int* launches);
+                               const int (&tr)[2], const int (&cu)[2][2], int* launches);
 
 void launch_combine(cudaStream_t st, int64_t n, const int64_t* cp_ptr, const int32_t* cp_pos, const double* cp_w,
                     const double* ylocal, const double* base, double* out);
