@@ -208,7 +208,7 @@ struct s2l_setup {
     CouplingUnit* d_cu[2] = {nullptr, nullptr};
     int32_t* d_crow[2] = {nullptr, nullptr};
     void *d_ccol[2] = {nullptr, nullptr}, *d_cval[2] = {nullptr, nullptr};
-    int cp_wide = 0;
+    int cp_wide = 0, max_tail = 0;
     void *d_linv = nullptr, *d_uinv = nullptr;
     bool need_gflags = false;
     std::vector<int> tr_first_h, cu_first_h[2];  // per subdomain, nsub+1 entries
@@ -1454,6 +1454,7 @@ LocalSolveArgs<Real> solve_args(s2l_work* w, int K, int mode)
     }
     a.tr_sub = s->d_tr_sub;
     a.tr_i = s->d_tr_i;
+    a.max_tail = s->max_tail;
     for (int f = 0; f < 2; ++f)
         a.cp[f] = Coupling<Real>{s->d_cu[f], s->d_crow[f], s->d_ccol[f], (const Real*)s->d_cval[f], s->cp_wide};
     a.linv = (const Real*)s->d_linv;
@@ -3195,6 +3196,8 @@ int s2l_gpu_setup_end(s2l_setup* s)
     s->tr_first_h[nsub] = (int)tr_sub.size();
     for (int f = 0; f < 2; ++f) s->cu_first_h[f][nsub] = (int)cpl[f].unit.size();
     s->cp_wide = max_nl > 65536;
+    s->max_tail = 0;
+    for (int i = 0; i < nsub; ++i) s->max_tail = std::max(s->max_tail, s->h_subs[i].n_local - s->h_subs[i].T);
     s->nloc = loc;
     if (!level) s->st_sparse_nnz = sparse_nnz;
     s->st_coupling_nnz = cpl[0].real + cpl[1].real;

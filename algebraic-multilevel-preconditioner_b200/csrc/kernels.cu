@@ -592,6 +592,114 @@ __device__ __forceinline__ Real pick(const Real (&acc)[K], int lane)
     return mine;
 }
 
+// The same products for four and more columns, where the x values of an entry are many times its own bytes.
+// One warp per row read them from L1 for every entry (16 columns, FP32, bubbles3d 100^3 / 64: 1.69 and 1.67 ms
+// for 480 MB each).  Here a CTA takes 8 R rows: chunks of x go to shared memory once for all of them (cp.async,
+// double buffered, 16-byte parts of neighbouring columns side by side, so neither side has bank conflicts), and
+// a warp keeps R rows' sums in registers, its lanes over the columns, so a shared load feeds R products.  The
+// lanes' sums are reduced and scattered in one butterfly.
+__device__ __forceinline__ void copy16_or_zero(void* dst, const void* src, bool ok)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(ok ? 16 : 0) : "memory");
+}
+
+template <typename Real, int K>
+struct TailTile {
+    static constexpr int R = K * (int)sizeof(Real) <= 64 ? 4 : 2;  // rows per warp: at most 64 registers of sums
+    static constexpr int ROWS = 8 * R;
+};
+
+template <typename Real, bool LOWER, int K>
+__global__ void __launch_bounds__(256, 2) tail_gemm_kernel(const LocalSolveArgs<Real> a, const Real* __restrict__ Minv,
+                                                           const Real* __restrict__ vin, Real* __restrict__ vout)
+{
+    constexpr int R = TailTile<Real, K>::R, ROWS = TailTile<Real, K>::ROWS;
+    constexpr int V = 16 / (int)sizeof(Real), C = K / V;  // 16-byte parts of a row of x
+    constexpr int CH = 128, U = CH / 32;
+    __shared__ uint4 xs[2][C][CH + 1];
+    const DevSub sd = a.subs[blockIdx.x];
+    const int s = sd.n_local - sd.T;
+    // longest rows first
+    const int rb = (LOWER ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y) * ROWS;
+    if (rb >= s) return;
+    const int lane = threadIdx.x & 31, i0 = rb + (threadIdx.x >> 5) * R;
+    const int64_t base = sd.loc_off + sd.T;
+    const Real* v = vin + base * K;
+    const int jb = LOWER ? 0 : rb, je = LOWER ? min(s, rb + ROWS) : s;
+    const int nch = (je - jb + CH - 1) / CH;
+    auto stage = [&](int t) {
+        const int j0 = jb + t * CH;
+        for (int e = threadIdx.x; e < CH * C; e += 256) {
+            const int j = e / C, c = e % C;
+            const bool ok = j0 + j < je;
+            copy16_or_zero(&xs[t & 1][c][j], v + (int64_t)(ok ? j0 + j : jb) * K + c * V, ok);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    Real acc[R * K];
+#pragma unroll
+    for (int q = 0; q < R * K; ++q) acc[q] = Real(0);
+    stage(0);
+    for (int t = 0; t < nch; ++t) {
+        const int j0 = jb + t * CH;
+        Real m[R][U];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = i0 + r;
+            const Real* row = Minv + sd.d_off + (int64_t)i * s;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int j = j0 + 32 * u + lane;
+                m[r][u] = i < s && (LOWER ? j <= i : j >= i && j < s) ? __ldg(row + j) : Real(0);
+            }
+        }
+        if (t + 1 < nch) {
+            stage(t + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const uint4 w = xs[t & 1][c][32 * u + lane];
+                Real x[V];
+                __builtin_memcpy(x, &w, 16);
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+#pragma unroll
+                    for (int q = 0; q < V; ++q) acc[r * K + c * V + q] += m[r][u] * x[q];
+            }
+        __syncthreads();  // before the buffer is staged again
+    }
+    // lane sums: half of the values go to the lane across at each step, until one or two are left
+    int first = 0, n = R * K;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool up = lane & o;
+#pragma unroll
+            for (int q = 0; q < R * K / 2; ++q) {
+                if (q >= n) break;
+                const Real send = up ? acc[q] : acc[q + n], keep = up ? acc[q + n] : acc[q];
+                acc[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+            first += up ? n : 0;
+        } else {
+            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+        }
+    }
+    constexpr int LEFT = R * K > 32 ? R * K / 32 : 1, SHARE = R * K < 32 ? 32 / (R * K) : 1;
+    if (lane & (SHARE - 1)) return;
+#pragma unroll
+    for (int q = 0; q < LEFT; ++q)
+        if (i0 + (first + q) / K < s) vout[(base + i0) * K + first + q] = acc[q];
+}
+
 // The couplings, K columns.  L: t(T+i) = b(T+i) - L(T+i, 0:T) y(0:T) of the tail rows; U: y(r) -= U(r, T:n)
 // x(T:n) of the sparse rows that have tail columns.  One warp per unit (CouplingUnit).
 //
@@ -1695,8 +1803,14 @@ cudaError_t launch_local_solve_k(cudaStream_t st, const LocalSolveArgs<Real>& a,
     if (tr[1] > 0) {
         const int g = (tr[1] + 7) / 8;
         nl += couple(std::true_type{});
-        tail_gemv_kernel<Real, true, K><<<g, 256, 0, st>>>(a, a.linv, a.ybuf, a.xbuf, tr[0], tr[1]);
-        tail_gemv_kernel<Real, false, K><<<g, 256, 0, st>>>(a, a.uinv, a.xbuf, a.ybuf, tr[0], tr[1]);
+        if constexpr (K >= 4) {  // (blocks solve every subdomain)
+            const dim3 gb(nblocks, (a.max_tail + TailTile<Real, K>::ROWS - 1) / TailTile<Real, K>::ROWS);
+            tail_gemm_kernel<Real, true, K><<<gb, 256, 0, st>>>(a, a.linv, a.ybuf, a.xbuf);
+            tail_gemm_kernel<Real, false, K><<<gb, 256, 0, st>>>(a, a.uinv, a.xbuf, a.ybuf);
+        } else {
+            tail_gemv_kernel<Real, true, K><<<g, 256, 0, st>>>(a, a.linv, a.ybuf, a.xbuf, tr[0], tr[1]);
+            tail_gemv_kernel<Real, false, K><<<g, 256, 0, st>>>(a, a.uinv, a.xbuf, a.ybuf, tr[0], tr[1]);
+        }
         nl += 2;
     }
     nl += couple(std::false_type{});

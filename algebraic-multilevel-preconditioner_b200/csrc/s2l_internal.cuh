@@ -152,6 +152,7 @@ struct LocalSolveArgs {
     const int32_t* tr_i;
     // 0: L(T+i, 0:T) (row i, columns: sparse rows), 1: U(r, T:n) (row r, columns: tail rows from 0 on)
     Coupling<Real> cp[2];
+    int max_tail;              // rows of the largest tail
     const Real* linv;          // inverse tails, row-major per subdomain
     const Real* uinv;
     const int32_t* gather;     // slot k -> index into `in` (global gather, or perm_in for a local input)
