@@ -597,7 +597,7 @@ __device__ __forceinline__ Real pick(const Real (&acc)[K], int lane)
 // for 480 MB each).  Here a CTA takes 8 R rows: chunks of x go to shared memory once for all of them (cp.async,
 // double buffered, 16-byte parts of neighbouring columns side by side, so neither side has bank conflicts), and
 // a warp keeps R rows' sums in registers, its lanes over the columns, so a shared load feeds R products.  The
-// lanes' sums are reduced and scattered in one butterfly.
+// lanes' sums are reduced and scattered in one butterfly.  The same case: 178 and 184 us (2.6 TB/s).
 __device__ __forceinline__ void copy16_or_zero(void* dst, const void* src, bool ok)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
@@ -707,7 +707,8 @@ __global__ void __launch_bounds__(256, 2) tail_gemm_kernel(const LocalSolveArgs<
 // for its values (10 bytes an entry in FP64, 6 in FP32; 12 and 8 with 32-bit columns and a load each before).
 // Two steps of a unit are in flight; consecutive lanes hold consecutive entries, whose columns mostly lie side by
 // side, so the gathers coalesce.  With more than 16 bytes of x per entry a lane reading all of them would
-// touch every sector several times (16 columns, FP32, bubbles3d 100^3 / 64: 587 us a coupling), so lanes share.
+// touch every sector several times, so lanes share.  bubbles3d 100^3 / 64, a coupling: 16 columns, FP32 587 us ->
+// 340; one column, FP64 174 and 200 us (L, U) -> 148 and 152 (811 MB each, 5.4 TB/s).
 template <bool ONCE>
 __device__ __forceinline__ uint4 load16(const uint4* p)  // ONCE: past L1, which is left to the gathers
 {
@@ -869,7 +870,7 @@ __global__ void __launch_bounds__(256) coupling_kernel(const LocalSolveArgs<Real
 }
 
 // Dense tail: out(T+i) = sum_j Minv(i, j) in(T+j), j <= i (lower) or j >= i (upper); warp per row,
-// K columns (Minv is read once for all of them).  The row is streamed with 16-byte loads (VEC
+// K columns, one or two (Minv is read once for both).  The row is streamed with 16-byte loads (VEC
 // entries per lane, two in flight per lane: 1 KB per warp), the few entries before the first
 // 16-byte boundary and after the last full vector one per lane.  Every column's sum runs in the same
 // order whatever K is.

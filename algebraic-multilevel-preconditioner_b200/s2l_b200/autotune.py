@@ -21,7 +21,8 @@ import numpy as np
 
 from . import capi
 
-# candidate values per option, searched in this order (the first value of each is the default)
+# candidate values per option, searched in this order; the first value of each stands for the default
+# (hop_us: 0.25 for dataflow sweeps, 2 for level sweeps) and is not built again
 SEARCH = (
     ("hop_us", (0.25, 0.1, 0.5, 1.0)),
     ("chain_block", (8, 4, 16)),
