@@ -34,17 +34,26 @@ __device__ __forceinline__ uint32_t cluster_rank()
 }
 
 // The barrier of every thread of the cluster (or of the CTA, alone), in two halves: stores before a
-// thread's arrival are seen after every other thread's wait
+// thread's arrival are seen after every other thread's wait.  The aligned forms want all lanes of a
+// warp at the same instruction, and the code before either half branches by lane (ragged loops over
+// the right-hand sides, partial copies): the warp comes together here first.
 template <bool CLUSTER>
 __device__ __forceinline__ void stage_arrive()
 {
-    if (CLUSTER) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (CLUSTER) {
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
 }
 template <bool CLUSTER>
 __device__ __forceinline__ void stage_wait()
 {
-    if (CLUSTER) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    else __syncthreads();
+    if (CLUSTER) {
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+        __syncthreads();
+    }
 }
 
 // the KC values of a slot to the CTA `rank` of the cluster
@@ -265,7 +274,6 @@ __global__ void __launch_bounds__(S2L_BS_LEVEL, 1) level_sweep_kernel(const Loca
         }
         // the next task's stage: arrive at once, prepare the next step, then wait
         const int st = (int)(dn.x >> 16);
-        __syncwarp();
         if (st > stage) stage_arrive<CLUSTER>();
         if (n > 0) next_step();
 #pragma unroll
