@@ -2818,12 +2818,14 @@ int s2l_gpu_setup_end(s2l_setup* s)
                 for (int64_t e = Us[i].rp[r]; e < Us[i].rp[r + 1]; ++e) cnt += Us[i].ci[e] >= Ts[i];
         // Entries a lane takes of a row: few where the rows are few, for warps and short chains; more where a
         // warp has many steps to do anyway, for less padding and fewer units.  Local solves in us with 2, 4, 16
-        // and 32: poisson2d 200^2 / 8 (0.3 steps a warp slot) 114, 117, 124, 135; bubbles3d 48^3 / 8 (10 steps)
-        // -, 280, 275, 293; 100^3 / 64 (109 steps) -, 1026, 1003, 997.
+        // and 32: poisson2d 200^2 / 8 (0.3 steps a warp slot) 114, 117, 124, 135; bubbles3d 30^3 / 8 in FP32 (0.6
+        // steps) 75, 79, 85, -, in FP64 (0.9 steps) 105, 104, 109, -; 32^3 / 8 (1.2 steps) 119, 112, 121, -;
+        // 40^3 / 32 (2 steps) 133, 131, 130, -; 48^3 / 8 (10 steps) -, 280, 275, 293; 100^3 / 64 (109 steps) -,
+        // 1026, 1003, 997.
         const double steps = (double)cnt / (128.0 * 32.0 * S2L_SMS);
         for (auto& c : cpl) {
             c.real_bytes = rs;
-            c.per_lane = steps >= 32.0 ? 32 : steps >= 4.0 ? 16 : 2;
+            c.per_lane = steps >= 32.0 ? 32 : steps >= 4.0 ? 16 : steps >= 0.75 ? 4 : 2;
         }
     }
     std::vector<std::vector<double>> Ltt(nsub), Utt(nsub);

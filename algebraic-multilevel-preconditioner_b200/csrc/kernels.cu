@@ -709,6 +709,11 @@ __global__ void __launch_bounds__(256, 2) tail_gemm_kernel(const LocalSolveArgs<
 // side, so the gathers coalesce.  With more than 16 bytes of x per entry a lane reading all of them would
 // touch every sector several times, so lanes share.  bubbles3d 100^3 / 64, a coupling: 16 columns, FP32 587 us ->
 // 340; one column, FP64 174 and 200 us (L, U) -> 148 and 152 (811 MB each, 5.4 TB/s).
+// A unit of few steps is a chain of loads: unit, subdomain and row, index, value, and the step itself.  With one and
+// two columns its first step is loaded beside the others and not after them, which small setups need (laplace3d
+// 27^3 / 6, L and U: 6.6 and 6.5 us -> 4.7 and 4.6; with a warp per row and 12-byte entries 5.1 and 6.3) and large
+// ones gain from (100^3 / 64, FP64: a local solve of one column 1004 -> 985 us, of two 1357 -> 1173).  Four columns
+// in FP32 lose by it (898 -> 922).
 template <bool ONCE>
 __device__ __forceinline__ uint4 load16(const uint4* p)  // ONCE: past L1, which is left to the gathers
 {
@@ -779,13 +784,23 @@ __global__ void __launch_bounds__(256) coupling_kernel(const LocalSolveArgs<Real
     const int64_t lo = sd.loc_off;
     const Real* x = a.ybuf + (TAIL_RHS ? lo : lo + sd.T) * K;
     const Col* col = (const Col*)cf.col;
-    // this lane's row, where it is, its index into the right-hand side and (one column) the value, ahead of the sum
+    // one and two columns: the first step needs the unit alone, so its loads go beside those of the subdomain
+    // and the rows
+    constexpr bool AHEAD = K <= 2;
+    CouplingStep<Real, Col> first;
+    if constexpr (AHEAD)
+        if (nsteps > 0) first.template load<true>(cf.val, col, cu.step, lane);
+    // this lane's row, where it is, its index into the right-hand side and (AHEAD) the values, before the sum
     const int ri = lane >> lg;
     const int row = ri < n ? cf.row[cu.row + ri] : -1;
     const int64_t k0 = row < 0 ? -1 : lo + (TAIL_RHS ? sd.T + row : row);
     const int g0 = TAIL_RHS && row >= 0 ? a.gather[k0] : 0;
-    Real b0 = Real(0);
-    if (K == 1 && row >= 0) b0 = TAIL_RHS ? (Real)a.in[g0] : a.ybuf[k0];
+    Real b0[AHEAD ? K : 1] = {};
+    if constexpr (AHEAD) {
+        if (row >= 0)
+#pragma unroll
+            for (int r = 0; r < K; ++r) b0[r] = TAIL_RHS ? (Real)a.in[(int64_t)g0 * K + r] : a.ybuf[k0 * K + r];
+    }
     // the right-hand side (L) or the row itself (U), less the sum of columns r and on
     auto put = [&](int64_t k, int g, int r, auto sum) {
         if (k < 0) return;
@@ -793,7 +808,7 @@ __global__ void __launch_bounds__(256) coupling_kernel(const LocalSolveArgs<Real
         Real* y = a.ybuf + k * K + r;
 #pragma unroll
         for (int q = 0; q < (int)(sizeof(sum.v) / sizeof(Real)); ++q)
-            y[q] = (K == 1 ? b0 : TAIL_RHS ? (Real)in[q] : y[q]) - sum.v[q];
+            y[q] = (AHEAD ? b0[AHEAD ? r + q : 0] : TAIL_RHS ? (Real)in[q] : y[q]) - sum.v[q];
     };
     const int G = 1 << lg;
     constexpr int P = K * (int)sizeof(Real) > 16 ? K * (int)sizeof(Real) / 16 : 1;
@@ -801,18 +816,29 @@ __global__ void __launch_bounds__(256) coupling_kernel(const LocalSolveArgs<Real
         Real acc[K];
 #pragma unroll
         for (int r = 0; r < K; ++r) acc[r] = Real(0);
-        CouplingStep<Real, Col> s0, s1;
-        int s = 0;
+        if constexpr (AHEAD) {
+            CouplingStep<Real, Col> s1;
 #pragma unroll 1
-        for (; s + 1 < nsteps; s += 2) {
-            s0.template load<true>(cf.val, col, cu.step + s, lane);
-            s1.template load<true>(cf.val, col, cu.step + s + 1, lane);
-            s0.template add<K>(x, acc);
-            s1.template add<K>(x, acc);
-        }
-        if (s < nsteps) {
-            s0.template load<true>(cf.val, col, cu.step + s, lane);
-            s0.template add<K>(x, acc);
+            for (int s = 0; s < nsteps; s += 2) {
+                if (s) first.template load<true>(cf.val, col, cu.step + s, lane);
+                if (s + 1 < nsteps) s1.template load<true>(cf.val, col, cu.step + s + 1, lane);
+                first.template add<K>(x, acc);
+                if (s + 1 < nsteps) s1.template add<K>(x, acc);
+            }
+        } else {
+            CouplingStep<Real, Col> s0, s1;
+            int s = 0;
+#pragma unroll 1
+            for (; s + 1 < nsteps; s += 2) {
+                s0.template load<true>(cf.val, col, cu.step + s, lane);
+                s1.template load<true>(cf.val, col, cu.step + s + 1, lane);
+                s0.template add<K>(x, acc);
+                s1.template add<K>(x, acc);
+            }
+            if (s < nsteps) {
+                s0.template load<true>(cf.val, col, cu.step + s, lane);
+                s0.template add<K>(x, acc);
+            }
         }
 #pragma unroll
         for (int r = 0; r < K; ++r)
