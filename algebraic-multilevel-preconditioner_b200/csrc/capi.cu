@@ -217,7 +217,8 @@ struct s2l_setup {
     int opt_tail_min = 64, opt_tail_max = 4096, opt_group = 0, opt_tail_rows = 0, opt_chain = S2L_CHAIN_DEFAULT, opt_block_width = 0,
         opt_tpr = 0, opt_epl = 4;
     int opt_level = -1;  // level sweeps: -1 where they are faster, 0 never, 1 wherever they fit
-    double opt_hop_us = 0.0, opt_bw_gbs = 6000.0;  // hop_us 0: the sweeps' default
+    double opt_hop_us = 0.0, opt_bw_gbs = 6000.0;
+    bool hop_given = false;  // opt_hop_us was set (any value, 0 too); else the sweeps' default
     std::atomic<int> opt_spin_limit{S2L_SPIN_LIMIT};  // polls of a sweep wait before it gives up
     std::atomic<int> opt_spin_sleep{S2L_SPIN_SLEEP_NS};  // back-off of a sweep poll that found a column not ready
     std::atomic<int> opt_sweep_pf{S2L_BATCH_CHUNKS};     // chunks a sweep warp hints into L2 ahead of its task
@@ -2719,7 +2720,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
     tm.real_bytes = (double)rs;
     // the tail split's model of the sweeps
     auto sweep_model = [&](bool lv, int ring) {
-        tm.hop_s = (s->opt_hop_us > 0.0 ? s->opt_hop_us : lv ? S2L_LEVEL_HOP_US : 0.25) * 1e-6;
+        tm.hop_s = (s->hop_given ? s->opt_hop_us : lv ? S2L_LEVEL_HOP_US : 0.25) * 1e-6;
         tm.chain = lv ? lcap : s->opt_chain;
         tm.fold = !lv;
         tm.index_bytes = lv ? 2.0 : 4.0;
@@ -3922,8 +3923,10 @@ int s2l_gpu_setup_option(s2l_setup* s, const char* name, double value)
     if (n == "tail_min") s->opt_tail_min = (int)value;
     else if (n == "tail_max") s->opt_tail_max = (int)value;
     else if (n == "tail_rows") s->opt_tail_rows = (int)value;
-    else if (n == "hop_us") s->opt_hop_us = value;
-    else if (n == "bw_gbs") s->opt_bw_gbs = value;
+    else if (n == "hop_us") {
+        s->opt_hop_us = value;
+        s->hop_given = true;
+    } else if (n == "bw_gbs") s->opt_bw_gbs = value;
     else if (n == "sweep_group") {
         const int g = (int)value;
         if (g != 0 && g != 8 && g != 16 && g != 32) return s->fail(S2L_ERR_BADARG, "sweep_group must be 0, 8, 16 or 32");

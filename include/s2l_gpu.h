@@ -182,8 +182,8 @@ int s2l_gpu_set_coarse(s2l_setup* s, int64_t n0, const int64_t* offsets, const d
  * chosen per subdomain to minimise 2 * hop_us * (sparse dependency levels) + bytes * nsub / bw_gbs.
  *   "tail_min" (rows, default 64), "tail_max" (default 4096): bounds of a non-empty tail;
  *   "tail_rows" (default 0 = cost model): force every subdomain's tail to this many rows;
- *   "hop_us" (default: 0.25 for dataflow sweeps, 2 for level sweeps), "bw_gbs" (default 6000): the
- *   cost model's parameters;
+ *   "hop_us" (default: 0.25 for dataflow sweeps, 2 for level sweeps; 0: by bytes alone), "bw_gbs"
+ *   (default 6000): the cost model's parameters;
  *   "level_sweeps" (default -1): the sparse sweeps go level by level with a thread-block cluster per
  *   subdomain and barriers (1: wherever x fits the shared memory), or row by row behind ready flags,
  *   one CTA per subdomain (0: dataflow sweeps); -1 chooses by the number of dependency levels.
