@@ -1109,6 +1109,9 @@ int upload_real(s2l_setup* s, void** dst, const std::vector<double>& v)
 }
 
 // ------------------------------------------------------------------------------ profiling
+// widest lane group of a row of the level sweeps
+int level_group(const s2l_setup* s) { return s->opt_group ? s->opt_group : 32; }
+
 // The layouts of the level sweeps, built and uploaded; mpos(i, f): factor positions of the entries of
 // factor f of subdomain i (refactorization) or nullptr, fsize(i): entries of its factor pattern.
 // S2L_ERR_STATE: x and s do not fit the shared memory (or 16-bit slots).
@@ -1116,7 +1119,7 @@ int build_level_layouts(s2l_setup* s, const std::vector<HostCsr>& Us, const std:
                         const std::function<const std::vector<int32_t>*(int, int)>& mpos,
                         const std::function<int64_t(int)>& fsize, int cap)
 {
-    const int nsub = s->nsub, warps = S2L_BS_LEVEL / 32, gmax = s->opt_group ? s->opt_group : 32;
+    const int nsub = s->nsub, warps = S2L_BS_LEVEL / 32, gmax = level_group(s);
     const bool track = mpos(0, 0) != nullptr;
     const size_t rs = s->real == S2L_REAL_F32 ? 4 : 8, sb = (size_t)level_step_bytes(rs);
     std::vector<int64_t> loc(nsub + 1, 0), fb(nsub + 1, 0);
@@ -2797,7 +2800,6 @@ int s2l_gpu_setup_end(s2l_setup* s)
         if (!level || s->opt_refactor) Ts = dataflow;
         if (level && !fits()) Ts = own;
     }
-    s->sweep_group = s->opt_group ? s->opt_group : 16;  // widest lane group of a sweep row
     const int nw = S2L_BS_SWEEP / 32;
     // pass 2: layouts
     int64_t loc = 0;
@@ -2859,7 +2861,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
         int code = S2L_OK;
     };
     std::vector<PreLayout> pre(nsub);
-    s->sweep_group = s->opt_group ? s->opt_group : 16;
+    s->sweep_group = s->opt_group ? s->opt_group : 16;  // widest lane group of a sweep row (dataflow sweeps)
     parallel_for(nsub, [&](int i) {
         HostSub& h = s->hs[i];
         if (h.amg) return;
@@ -2903,6 +2905,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
             return rc;
         }
     }
+    if (level) s->sweep_group = level_group(s);
     if (!level) parallel_for(nsub, [&](int i) {
         HostSub& h = s->hs[i];
         if (h.amg) return;

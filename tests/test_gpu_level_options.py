@@ -26,3 +26,13 @@ def test_hop_us_zero_splits_by_bytes_alone(ctx, level):
         g.close()
     assert got[0] == got[1]
     assert got[0][0] < got[2][0]  # levels that cost nothing need no tail
+
+
+def test_sweep_group_statistic(ctx):
+    """The widest lane group of the sweeps that run: 16 (dataflow) or 32 (level) unless set."""
+    from s2l_b200.capi import GpuSetup
+    _, st = small_setup("poisson2d", nx=61, nsub=3)
+    for options, group in (({"level_sweeps": 1}, 32), ({"level_sweeps": 0}, 16), ({"level_sweeps": 1, "sweep_group": 8}, 8)):
+        g = GpuSetup(ctx, st, options=options)
+        assert g.stat("sweep_group") == group, options
+        g.close()
