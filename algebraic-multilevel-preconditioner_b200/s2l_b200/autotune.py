@@ -10,6 +10,9 @@ same host setup with candidate values, times each with CUDA events on the device
 kernel timers around the local solve and the SpMV of ``s2l_gpu_apply_block`` / ``s2l_gpu_spmv``),
 and keeps the fastest: a coordinate search, one option at a time, starting from the defaults.
 
+Setups with level sweeps have other defaults and other values worth a try than those with dataflow
+sweeps: ``LEVEL_SEARCH`` is searched when the default setup has them.  Both lists try the other kind.
+
 The objective is the time of one Arnoldi step's layout-dependent kernels for a block of ``k``
 right-hand sides: one block local solve plus ``spmv_per_step`` products with A.
 """
@@ -21,12 +24,22 @@ import numpy as np
 
 from . import capi
 
-# candidate values per option, searched in this order; the first value of each stands for the default
-# (hop_us: 0.25 for dataflow sweeps, 2 for level sweeps) and is not built again
+# candidate values per option, searched in this order; the first value of each is the default and is not
+# built again
 SEARCH = (
     ("hop_us", (0.25, 0.1, 0.5, 1.0)),
     ("chain_block", (8, 4, 16)),
     ("sweep_group", (16, 32, 8)),
+    ("level_sweeps", (-1, 1)),
+    ("spmv_tpr", (0, 1, 2, 4)),
+    ("sweep_prefetch", (8, 16, 24)),
+)
+# the same for setups with level sweeps (chain_block 8 and more give the same blocks of 64 rows)
+LEVEL_SEARCH = (
+    ("hop_us", (2.0, 1.0, 4.0)),
+    ("chain_block", (8, 4)),
+    ("sweep_group", (32, 16)),
+    ("level_sweeps", (-1, 0)),
     ("spmv_tpr", (0, 1, 2, 4)),
     ("sweep_prefetch", (8, 16, 24)),
 )
@@ -35,7 +48,8 @@ RUNTIME = ("sweep_prefetch", "spin_sleep_ns")
 
 
 def measure(g: capi.GpuSetup, k: int, reps: int, rng) -> dict:
-    """Average device time [ms] of one block local solve of k columns and of one product with A."""
+    """Average device time [ms] of one block local solve of k columns and of one product with A (and
+    the CTAs per subdomain of the setup's level sweeps, 0: dataflow sweeps)."""
     R = rng.uniform(-1.0, 1.0, (k, g.n))
     x = rng.uniform(-1.0, 1.0, g.n)
     g.apply_block(R)  # warm-up (and the block buffers)
@@ -48,13 +62,15 @@ def measure(g: capi.GpuSetup, k: int, reps: int, rng) -> dict:
     sp_ms, sp_n = g.profile_get("spmv")
     g.profile(())
     # the deflated apply runs a product with A of its own: keep only the spmv calls' own share
-    return {"local_solve_ms": ls_ms / max(ls_n, 1), "spmv_ms": sp_ms / max(sp_n, 1)}
+    return {"local_solve_ms": ls_ms / max(ls_n, 1), "spmv_ms": sp_ms / max(sp_n, 1),
+            "level_sweeps": int(g.stat("level_sweeps"))}
 
 
 def tune(ctx: capi.Context, st, k: int = 4, reps: int = 5, spmv_per_step: int = 2, base=None, search=SEARCH,
-         seed: int = 0):
+         seed: int = 0, level_search=None):
     """Coordinate search over `search`; returns (the fastest GpuSetup, report).  `base`: options
-    every candidate keeps (e.g. {"refactor": 1})."""
+    every candidate keeps (e.g. {"refactor": 1}).  `level_search`: searched instead when the default
+    setup has level sweeps (None: LEVEL_SEARCH in place of SEARCH, any other `search` as it is)."""
     rng = np.random.default_rng(seed)
     base = dict(base or {})
     current = {}
@@ -92,6 +108,10 @@ def tune(ctx: capi.Context, st, k: int = 4, reps: int = 5, spmv_per_step: int = 
 
     trial({})
     default_t = best_t
+    if level_search is None and search is SEARCH:
+        level_search = LEVEL_SEARCH
+    if level_search is not None and best_m.get("level_sweeps", 0) > 0:
+        search = level_search
     for name, values in search:
         chosen = current.get(name)
         for v in values[1:]:

@@ -285,9 +285,12 @@ class Replicas:
 
 
 # the autotuner's search in the benchmark: a reduced set of candidates (every candidate is a device
-# setup of the 100^3 workload), the first value of each option the default
+# setup of the 100^3 workload), the first value of each option the default; the second list when the
+# default setup has level sweeps
 TUNE_SEARCH = (("hop_us", (0.25, 0.1, 0.5)), ("chain_block", (8, 16)), ("sweep_group", (16, 32)),
                ("spmv_tpr", (0, 1)), ("sweep_prefetch", (8, 16, 24)))
+TUNE_LEVEL_SEARCH = (("hop_us", (2.0, 1.0, 4.0)), ("sweep_group", (32, 16)), ("level_sweeps", (-1, 0)),
+                     ("spmv_tpr", (0, 1)), ("sweep_prefetch", (8, 16, 24)))
 
 
 def workload_desc(w, overlap) -> str:
@@ -487,7 +490,8 @@ def run_ours(a):
         # the mixed setup's layout chosen by timing candidates on the device (4-column blocks, the
         # width of the headline's blocks); the FP64 setup takes the same options
         from s2l_b200 import autotune
-        g32, tuning = autotune.tune(ctx, st32, k=4, reps=3, base=layout, search=TUNE_SEARCH)
+        g32, tuning = autotune.tune(ctx, st32, k=4, reps=3, base=layout, search=TUNE_SEARCH,
+                                    level_search=TUNE_LEVEL_SEARCH)
         layout = dict(layout, **tuning["chosen"])
     else:
         g32 = capi.GpuSetup(ctx, st32, options=layout)
