@@ -51,6 +51,7 @@ struct s2l_ctx {
     size_t used = 0;
     std::string err;
     std::mutex mu;
+    std::vector<s2l_setup*> spares;  // setups that hold a second layout (s2l_setup::spare; under mu)
     s2l_serve* serve = nullptr;
     // device address of the static scratch of s2l_gpu_coarse_apply_noalloc, looked up by the first
     // such call on this context (with its device current); a context created after a reset of the
@@ -200,7 +201,12 @@ struct s2l_setup {
         int64_t *boff[2] = {nullptr, nullptr}, *wsrc[2] = {nullptr, nullptr}, *wpos[2] = {nullptr, nullptr};
         int64_t nblk[2] = {0, 0};
     } lay[2];
-    int nlay = 0;
+    std::atomic<int> nlay{0};
+    // The memory of layout 1, which only makes blocks faster: given back when an allocation of the
+    // context would fail otherwise and no call runs on the setup (under ctx->mu)
+    std::vector<void*> spare;
+    size_t spare_bytes = 0;
+    int active = 0;  // calls that may launch on the layouts
     void* d_val[2] = {nullptr, nullptr};
     void* d_dinv[2] = {nullptr, nullptr};
     int32_t *d_tr_sub = nullptr, *d_tr_i = nullptr;
@@ -420,26 +426,77 @@ namespace {
 
 int check_err(s2l_work* w);
 
-int dev_alloc(s2l_setup* s, void** p, size_t bytes)
+// Frees the second layout of a setup that no call runs on; false: there is none.
+bool give_back_spare(s2l_ctx* c)
+{
+    std::vector<void*> gone;
+    size_t bytes = 0;
+    {
+        std::lock_guard<std::mutex> g(c->mu);
+        const auto it = std::find_if(c->spares.begin(), c->spares.end(), [](const s2l_setup* s) { return s->active == 0; });
+        if (it == c->spares.end()) return false;
+        s2l_setup* s = *it;
+        c->spares.erase(it);
+        gone.swap(s->spare);
+        bytes = s->spare_bytes;
+        s->spare_bytes = 0;
+        s->nlay = 1;
+        s->lay[1] = {};
+    }
+    cudaDeviceSynchronize();  // (a call that failed may have left kernels behind)
+    for (void* p : gone) cudaFree(p);
+    std::lock_guard<std::mutex> g(c->mu);
+    c->used -= std::min(c->used, bytes);
+    return true;
+}
+
+thread_local size_t t_refused = 0;  // size of this thread's last allocation over the budget (0: cudaMalloc failed)
+
+// After a refused allocation: whether second layouts that calls are using would make room for it.  They come
+// free when those calls end; an allocation waits for that, S2L_SPARE_WAIT_S seconds at most.
+bool spare_would_do(s2l_ctx* c)
+{
+    std::lock_guard<std::mutex> g(c->mu);
+    size_t sum = 0;
+    for (const s2l_setup* s : c->spares) sum += s->spare_bytes;
+    return sum > 0 && t_refused > 0 && c->used - std::min(c->used, sum) + t_refused <= c->budget;
+}
+
+// device memory within the context's budget; second layouts that idle setups hold make room for it
+int ctx_alloc(s2l_ctx* c, void** p, size_t bytes)
 {
     *p = nullptr;
-    if (bytes == 0) bytes = 16;
-    {
-        std::lock_guard<std::mutex> g(s->ctx->mu);
-        if (s->ctx->budget && s->ctx->used + bytes > s->ctx->budget) {
-            s->ctx->err = "HBM budget exceeded: need " + std::to_string(s->ctx->used + bytes) + " of " +
-                          std::to_string(s->ctx->budget) + " bytes";
-            return S2L_ERR_OOM;
+    do {
+        {
+            std::lock_guard<std::mutex> g(c->mu);
+            if (c->budget && c->used + bytes > c->budget) {
+                c->err = "HBM budget exceeded: need " + std::to_string(c->used + bytes) + " of " + std::to_string(c->budget) +
+                         " bytes";
+                t_refused = bytes;
+                continue;
+            }
+            c->used += bytes;
         }
-        s->ctx->used += bytes;
-    }
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) {
-        std::lock_guard<std::mutex> g(s->ctx->mu);
-        s->ctx->used -= bytes;
-        s->ctx->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
-        return S2L_ERR_OOM;
-    }
+        t_refused = 0;
+        const cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaSuccess) return S2L_OK;
+        (void)cudaGetLastError();  // reported here, not by the next launch
+        std::lock_guard<std::mutex> g(c->mu);
+        c->used -= bytes;
+        c->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+    } while (give_back_spare(c));
+    return S2L_ERR_OOM;
+}
+
+int dev_alloc(s2l_setup* s, void** p, size_t bytes)
+{
+    if (bytes == 0) bytes = 16;
+    const auto deadline = std::chrono::steady_clock::now() + std::chrono::seconds(S2L_SPARE_WAIT_S);
+    int rc;
+    while ((rc = ctx_alloc(s->ctx, p, bytes)) == S2L_ERR_OOM && spare_would_do(s->ctx) &&
+           std::chrono::steady_clock::now() < deadline)
+        std::this_thread::sleep_for(std::chrono::milliseconds(2));  // (no lock is held here)
+    RET_IF(rc);
     s->allocs.push_back(*p);
     s->bytes += bytes;
     return S2L_OK;
@@ -1296,12 +1353,21 @@ int build_level_layouts(s2l_setup* s, const std::vector<HostCsr>& Us, const std:
             CUDA_OK(s, cudaStreamSynchronize(s->setup_stream));
             q.clear();
         }
-        s->nlay = v + 1;
+        if (v == 0) s->nlay = 1;
         return S2L_OK;
     };
     for (int v = 0; v < nlay; ++v) {
         const size_t mark = s->allocs.size(), before = s->bytes;
         const int rc = build(v);
+        if (rc == S2L_OK && v == 1) {
+            std::lock_guard<std::mutex> g(s->ctx->mu);
+            s->spare.assign(s->allocs.begin() + (long)mark, s->allocs.end());
+            s->spare_bytes = s->bytes - before;
+            s->allocs.resize(mark);
+            s->bytes = before;
+            s->nlay = 2;
+            s->ctx->spares.push_back(s);
+        }
         if (rc == S2L_OK) continue;
         if (v == 0 || (rc != S2L_ERR_OOM && rc != S2L_ERR_STATE)) return rc;
         // no memory for a second layout: blocks run on the first
@@ -1326,25 +1392,8 @@ int check_ready(s2l_setup* s)
 
 int work_alloc(s2l_work* w, void** p, size_t bytes)
 {
-    *p = nullptr;
     if (bytes == 0) bytes = 16;
-    s2l_ctx* c = w->s->ctx;
-    {
-        std::lock_guard<std::mutex> g(c->mu);
-        if (c->budget && c->used + bytes > c->budget) {
-            c->err = "HBM budget exceeded: need " + std::to_string(c->used + bytes) + " of " + std::to_string(c->budget) +
-                     " bytes";
-            return S2L_ERR_OOM;
-        }
-        c->used += bytes;
-    }
-    const cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) {
-        std::lock_guard<std::mutex> g(c->mu);
-        c->used -= bytes;
-        c->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
-        return S2L_ERR_OOM;
-    }
+    RET_IF(ctx_alloc(w->s->ctx, p, bytes));
     w->allocs.push_back(*p);
     w->alloc_bytes.push_back(bytes);
     w->bytes += bytes;
@@ -1446,8 +1495,8 @@ LocalSolveArgs<Real> solve_args(s2l_work* w, int K, int mode)
     a.gather = mode == 2 ? s->d_pin : s->d_gin;
     a.K = K;
     a.KC = std::min(K, s->kc_max);
-    if (s->nlay > 0) {
-        const auto& y = s->lay[K > 1 ? s->nlay - 1 : 0];
+    if (const int nlay = s->nlay; nlay > 0) {
+        const auto& y = s->lay[K > 1 ? nlay - 1 : 0];
         for (int f = 0; f < 2; ++f) a.lf[f] = level_factor<Real>(y, f);
         a.cs = y.cs;
         a.slots = y.slots;
@@ -1951,9 +2000,11 @@ int invert_tails(s2l_setup* s, const std::vector<std::vector<double>>& Ltt, cons
     if (max_sz == 0) return S2L_OK;
     double *dA = nullptr, *dB = nullptr;
     const size_t mb = (size_t)max_sz * max_sz * sizeof(double);
-    if (cudaMalloc(&dA, mb) != cudaSuccess || cudaMalloc(&dB, mb) != cudaSuccess) {
+    while (cudaMalloc(&dA, mb) != cudaSuccess || cudaMalloc(&dB, mb) != cudaSuccess) {
+        (void)cudaGetLastError();
         cudaFree(dA);
-        return s->fail(S2L_ERR_OOM, "no device memory for the tail inversion");
+        dA = nullptr;
+        if (!give_back_spare(s->ctx)) return s->fail(S2L_ERR_OOM, "no device memory for the tail inversion");
     }
     cublasHandle_t hb = nullptr;
     int rc = S2L_OK;
@@ -2114,6 +2165,7 @@ struct Lease {
         }
         std::unique_lock<std::mutex> g(s->wmu);
         const auto deadline = std::chrono::steady_clock::now() + std::chrono::seconds(S2L_ADMIT_WAIT_S);
+        const auto spare_deadline = std::chrono::steady_clock::now() + std::chrono::seconds(S2L_SPARE_WAIT_S);
         auto take = [&](size_t i) -> int {  // reserve workspace i and prepare it (lock released meanwhile)
             s->busy[i] = 1;
             s2l_work* cand = s->works[i];
@@ -2152,12 +2204,20 @@ struct Lease {
             }
             bool anybusy = false;
             for (char b : s->busy) anybusy = anybusy || b;
+            if (!anybusy && spare_would_do(s->ctx) && std::chrono::steady_clock::now() < spare_deadline) {
+                s->wcv.wait_for(g, std::chrono::milliseconds(2));
+                continue;
+            }
             if (!anybusy || s->wcv.wait_until(g, deadline) == std::cv_status::timeout) {
                 rc = S2L_ERR_OOM;  // the message of the failed allocation stays in last_error
                 return;
             }
         }
         w = s->works[idx];
+        {
+            std::lock_guard<std::mutex> a(s->ctx->mu);
+            ++s->active;
+        }
         // another workspace's stream starts after the work already queued on the caller's stream
         if (idx != 0 && s->user_stream) {
             if (cudaEventRecord(w->join, s->user_stream) != cudaSuccess ||
@@ -2168,6 +2228,10 @@ struct Lease {
     ~Lease()
     {
         if (idx < 0) return;
+        {
+            std::lock_guard<std::mutex> a(s->ctx->mu);
+            --s->active;
+        }
         {
             std::lock_guard<std::mutex> g(s->wmu);
             s->busy[idx] = 0;
@@ -3548,7 +3612,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
         for (int kc = 2; kc <= 4; kc *= 2)
             if ((((slots * kc * rs) + 15) & ~(size_t)15) + ((slots + 15) & ~(size_t)15) <= smem_cap)
                 s->kc_max = kc;
-    if (level) s->kc_max = s->lay[s->nlay - 1].kc_max;
+    if (level) s->kc_max = s->lay[0].kc_max;  // (as many slots in layout 1)
     CUDA_OK(s, cudaStreamSynchronize(s->setup_stream));
     // host staging no longer needed
     s->A.ci = {};  // the row pointers stay: s2l_gpu_update_matrix recomputes the row sums with them
@@ -3576,6 +3640,13 @@ int s2l_gpu_setup_destroy(s2l_setup* s)
     cudaSetDevice(s->ctx->device);
     for (s2l_work* w : s->works) work_destroy(w);
     if (s->setup_stream) cudaStreamSynchronize(s->setup_stream);
+    {
+        std::lock_guard<std::mutex> g(s->ctx->mu);
+        auto& q = s->ctx->spares;
+        q.erase(std::remove(q.begin(), q.end(), s), q.end());
+        s->allocs.insert(s->allocs.end(), s->spare.begin(), s->spare.end());
+        s->bytes += s->spare_bytes;
+    }
     for (void* p : s->allocs) cudaFree(p);
     {
         std::lock_guard<std::mutex> g(s->ctx->mu);
@@ -3890,6 +3961,16 @@ int s2l_gpu_refactor(s2l_setup* s, const double* val, int ptr_kind)
         if (b) return s->fail(S2L_ERR_STATE, "refactor while a solve-phase call runs on the setup");
     if (s->pending.load() > 0) return s->fail(S2L_ERR_STATE, "refactor while solves are queued on the setup");
     if (cudaSetDevice(s->ctx->device) != cudaSuccess) return s->fail(S2L_ERR_CUDA, "cudaSetDevice failed");
+    struct InUse {  // the layouts stay as they are meanwhile
+        s2l_setup* s;
+        void add(int d)
+        {
+            std::lock_guard<std::mutex> a(s->ctx->mu);
+            s->active += d;
+        }
+        explicit InUse(s2l_setup* s_) : s(s_) { add(1); }
+        ~InUse() { add(-1); }
+    } in_use(s);
     return refactor_run(s, val, ptr_kind);
 }
 
@@ -3899,6 +3980,8 @@ int s2l_gpu_setup_bytes(const s2l_setup* s, size_t* bytes)
     std::lock_guard<std::mutex> g(s->wmu);
     size_t b = s->bytes;
     for (const s2l_work* w : s->works) b += w->bytes;
+    std::lock_guard<std::mutex> a(s->ctx->mu);
+    b += s->spare_bytes;
     *bytes = b;
     return S2L_OK;
 }
@@ -3978,6 +4061,7 @@ int s2l_gpu_setup_stat(const s2l_setup* s, const char* name, double* value)
     else if (n == "sweep_group") *value = (double)s->sweep_group;
     else if (n == "smem_bytes") *value = (double)s->smem_bytes;
     else if (n == "level_sweeps") *value = (double)(s->nlay > 0 ? s->lay[0].cs : 0);
+    else if (n == "level_layouts") *value = (double)s->nlay.load();
     else if (n == "levels_max") *value = (double)s->st_levels_max;
     else if (n == "chain_blocks") *value = (double)s->st_blocks;
     else if (n == "sweep_tasks") *value = (double)s->st_tasks;

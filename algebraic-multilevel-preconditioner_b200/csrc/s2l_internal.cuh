@@ -31,6 +31,7 @@
 #define S2L_CHAIN_MAX 16
 #define S2L_SWEEP_SMEM_CAP (227 * 1024 - 64)  // dynamic shared memory of a sweep CTA, at most
 #define S2L_ADMIT_WAIT_S 600   // longest wait of a call for a free workspace when the HBM budget is full
+#define S2L_SPARE_WAIT_S 2     // longest wait of an allocation for another setup's second layout while calls use it
 #ifndef S2L_SPIN_SLEEP_NS
 #define S2L_SPIN_SLEEP_NS 0   // pause of a sweep warp after a poll that found a column not ready (ns; 0 = none)
 #endif

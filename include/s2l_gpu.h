@@ -254,7 +254,9 @@ int s2l_gpu_refactor(s2l_setup* s, const double* val, int ptr_kind);
 int s2l_gpu_setup_bytes(const s2l_setup* s, size_t* bytes);
 /* Layout statistics after setup_end: "sparse_nnz", "coupling_nnz", "dense_entries", "tail_rows",
    "sweep_group", "smem_bytes", "level_sweeps" (CTAs per subdomain of the level sweeps; 0: dataflow
-   sweeps), "levels_max" / "levels_mean" (dependency levels of a sparse sweep,
+   sweeps), "level_layouts" (2: blocks of columns have a layout of their own; it is given back, at any
+   time no call runs on the setup, when an allocation of the context needs its memory, and blocks then
+   run on layout 1, their sums in another order), "levels_max" / "levels_mean" (dependency levels of a sparse sweep,
    largest and mean over subdomains and both factors), "chain_blocks", "sweep_tasks" and
    "sweep_padding" (padding entries of the lane-interleaved task layout), both factors;
    "local_solve_column_bytes": the part of s2l_gpu_local_solve_bytes that each further right-hand
