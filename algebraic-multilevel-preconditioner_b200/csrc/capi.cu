@@ -2715,64 +2715,70 @@ int wait_runners_gone(s2l_setup* s)
 
 }  // namespace
 
-extern "C" {
+namespace {
 
-int s2l_gpu_setup_end(s2l_setup* s)
+// Bytes of device memory left to the context (its budget or the device's memory)
+double memory_left(s2l_ctx* c)
 {
-    if (!s) return S2L_ERR_BADARG;
-    if (s->ended) return s->fail(S2L_ERR_STATE, "setup_end called twice");
-    if (!s->have_A) return s->fail(S2L_ERR_STATE, "set_matrix was not called");
-    if (cudaSetDevice(s->ctx->device) != cudaSuccess) return S2L_ERR_CUDA;
+    size_t free_b = 0, total = 0;
+    if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) return 0.0;
+    std::lock_guard<std::mutex> g(c->mu);
+    const double left = c->budget > c->used ? (double)(c->budget - c->used) : 0.0;
+    return c->budget ? std::min(left, (double)free_b) : (double)free_b;
+}
+
+// handles, streams and events of the refactorization plan
+void refactor_release(s2l_setup* s)
+{
+    for (int q = 0; q < s2l_setup::Refac::RF_STREAMS; ++q) {
+        if (s->rf.tsolver[q]) cusolverDnDestroy(s->rf.tsolver[q]);
+        if (s->rf.tstream[q]) cudaStreamDestroy(s->rf.tstream[q]);
+    }
+    for (auto e : s->rf.tev)
+        if (e) cudaEventDestroy(e);
+}
+
+// Undoes setup_layouts: the device memory taken since `mark` allocations and `before` bytes, and what was set
+void drop_layouts(s2l_setup* s, size_t mark, size_t before)
+{
+    cudaStreamSynchronize(s->setup_stream);
+    size_t bytes = s->bytes - before;
+    {
+        std::lock_guard<std::mutex> g(s->ctx->mu);
+        auto& q = s->ctx->spares;
+        q.erase(std::remove(q.begin(), q.end(), s), q.end());
+        s->allocs.insert(s->allocs.end(), s->spare.begin(), s->spare.end());
+        s->spare.clear();
+        bytes += s->spare_bytes;
+        s->spare_bytes = 0;
+    }
+    for (size_t i = mark; i < s->allocs.size(); ++i) cudaFree(s->allocs[i]);
+    s->allocs.resize(mark);
+    s->bytes = before;
+    {
+        std::lock_guard<std::mutex> g(s->ctx->mu);
+        s->ctx->used -= std::min(s->ctx->used, bytes);
+    }
+    refactor_release(s);
+    s->rf = s2l_setup::Refac{};
+    for (auto& y : s->lay) y = {};
+    s->nlay = 0;
+    s->need_gflags = false;
+    s->st_levels_max = s->st_levels_sum = s->st_sparse_nnz = s->st_pad = s->st_tasks = s->st_blocks = 0;
+}
+
+// The layouts of the local solves, the coarse space, the refactorization plan and workspace 0, from the factors
+// (h.L and the full U of every subdomain, kept on the host when `keep` is set).  smallest: dataflow sweeps
+// and the narrowest couplings, whatever is faster.
+int setup_layouts(s2l_setup* s, std::vector<HostCsr>& Us, bool smallest, bool keep)
+{
     const int nsub = s->nsub;
-    if (s->local_kind == 1 && s->opt_refactor)
-        return s->fail(S2L_ERR_BADARG, "the option refactor needs exact local factors");
-    // ---- ownership checks: contiguous ranges covering [0, n)
-    {
-        int64_t next = 0;
-        for (int i = 0; i < nsub; ++i) {
-            if (!s->hs[i].set) return s->fail(S2L_ERR_STATE, "subdomain " + std::to_string(i) + " was not added");
-            if (s->hs[i].begin != next) return s->fail(S2L_ERR_BADARG, "owned ranges must be contiguous in subdomain order");
-            next += s->hs[i].n_owned;
-        }
-        if (next != s->n) return s->fail(S2L_ERR_BADARG, "owned ranges do not cover [0, n)");
-    }
-    if (s->coarse != S2L_COARSE_NONE) {
-        if (!s->have_coarse) return s->fail(S2L_ERR_STATE, "set_coarse was not called");
-        if (s->coff[0] != 0 || s->coff[nsub] != s->n0) return s->fail(S2L_ERR_BADARG, "coarse offsets inconsistent with n0");
-        for (int i = 0; i < nsub; ++i)
-            if (s->coff[i + 1] - s->coff[i] != s->hs[i].m)
-                return s->fail(S2L_ERR_BADARG, "coarse offsets do not match the basis sizes");
-    }
     const bool boolean = s->pou == S2L_POU_BOOLEAN;
-    s->need_copies = !(boolean && s->one_level == S2L_ONE_LEVEL_RAS);
-
-    // ---- global matrix
-    {
-        std::vector<int32_t> rp(s->n + 1);
-        for (int64_t r = 0; r <= s->n; ++r) rp[r] = (int32_t)s->A.rp[r];
-        s->nnz = s->A.rp[s->n];
-        RET_IF(upload(s, &s->d_rp, rp));
-        RET_IF(upload(s, &s->d_ci, s->A.ci));
-        RET_IF(upload(s, &s->d_av, s->A.v));
-        std::vector<double> rowsum(s->n, 0.0);  // A 1, summed in row order as a CSR product does
-        for (int64_t r = 0; r < s->n; ++r)
-            for (int64_t e = s->A.rp[r]; e < s->A.rp[r + 1]; ++e) rowsum[r] += s->A.v[e];
-        RET_IF(upload(s, &s->d_rowsum, rowsum));
-        const double avg = (double)s->nnz / (double)s->n;
-        // lanes per row for about four entries per lane, between 2 and 32 (each lane with four
-        // entries in flight: on a 7-point matrix 2 lanes per row beat the chunk mode, a warp per 32
-        // rows with coalesced entry loads, spmv_tpr 1, by 1.3x for one column and 1.5x for four)
-        int tpr = 2;
-        while (tpr < 32 && tpr * 4 < avg) tpr *= 2;
-        s->tpr = s->opt_tpr ? s->opt_tpr : tpr;
-    }
-
     // ---- per-subdomain factor split, sweep layouts and index maps
     s->h_subs.resize(nsub);
     const size_t rs = s->real == S2L_REAL_F32 ? 4 : 8;
-    // pass 1: full U of every subdomain and its tail split
-    std::vector<HostCsr> Us(nsub);
     std::vector<int> Ts(nsub);
+    for (int i = 0; i < nsub; ++i) Ts[i] = s->hs[i].n_local();  // (AMG: no factors, the whole local space)
     s2l_tail_model tm;
     tm.force_rows = s->opt_tail_rows;
     tm.tail_min = s->opt_tail_min;
@@ -2780,7 +2786,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
     // Level sweeps, unless the chain blocks are off: without blocks the levels are single rows by the
     // hundred and a barrier for each costs more than the dataflow sweeps' flags.  (The layouts below
     // still fall back to dataflow sweeps when x and s do not fit the shared memory.)
-    bool level = s->local_kind == 0 && s->opt_chain > 1 && s->opt_level != 0;
+    bool level = !smallest && s->local_kind == 0 && s->opt_chain > 1 && s->opt_level != 0;
     const int lcap = std::min(8 * s->opt_chain, S2L_LEVEL_CAP);
     tm.bw = s->opt_bw_gbs * 1e9;
     tm.nsub = nsub;
@@ -2795,42 +2801,6 @@ int s2l_gpu_setup_end(s2l_setup* s)
         tm.slot_bytes = lv ? rs : rs + 1.0;
         tm.smem_cap = (double)S2L_SWEEP_SMEM_CAP - (lv ? (double)level_smem_bytes(rs, 1024, 1, ring) : 0.0);
     };
-    // per subdomain and independent of the others: on several host threads
-    std::vector<char> ldlt_bad(nsub, 0);
-    parallel_for(nsub, [&](int i) {
-        HostSub& h = s->hs[i];
-        const int nl = h.n_local();
-        if (h.amg) {  // no factors: the whole local space is "sparse part" without a tail
-            Ts[i] = nl;
-            return;
-        }
-        if (h.kind == S2L_FACTOR_LU) {
-            Us[i] = std::move(h.U);
-        } else {
-            Us[i] = transpose_lower(h.L, nl, nullptr);
-            if (h.kind == S2L_FACTOR_LDLT) {
-                bool missing = false;
-                for (int r = 0; r < nl; ++r) {
-                    bool f = false;
-                    for (int64_t e = Us[i].rp[r]; e < Us[i].rp[r + 1]; ++e) {
-                        if (Us[i].ci[e] == r) {
-                            Us[i].v[e] = h.d[r];
-                            f = true;
-                        } else {
-                            Us[i].v[e] *= h.d[r];
-                        }
-                    }
-                    missing = missing || !f;
-                }
-                if (missing) {
-                    ldlt_bad[i] = 1;
-                    return;
-                }
-            }
-        }
-    });
-    for (int i = 0; i < nsub; ++i)
-        if (ldlt_bad[i]) return s->fail(S2L_ERR_BADARG, "LDLT: L must store its unit diagonal");
     std::vector<int> levels(nsub, 0);
     int deepest = 0;  // levels of the split's deepest subdomain
     auto fits = [&]() {
@@ -2892,7 +2862,7 @@ int s2l_gpu_setup_end(s2l_setup* s)
         const double steps = (double)cnt / (128.0 * 32.0 * S2L_SMS);
         for (auto& c : cpl) {
             c.real_bytes = rs;
-            c.per_lane = steps >= 32.0 ? 32 : steps >= 4.0 ? 16 : steps >= 0.75 ? 4 : 2;
+            c.per_lane = steps >= 32.0 ? 32 : smallest || steps >= 4.0 ? 16 : steps >= 0.75 ? 4 : 2;
         }
     }
     std::vector<std::vector<double>> Ltt(nsub), Utt(nsub);
@@ -3260,8 +3230,10 @@ int s2l_gpu_setup_end(s2l_setup* s)
         Dall.insert(Dall.end(), h.D.begin(), h.D.end());
         bytes += (double)sz * (sz + 1) * rs;
         loc += nl;
-        h.L = HostCsr();
-        Us[i] = HostCsr();
+        if (!keep) {
+            h.L = HostCsr();
+            Us[i] = HostCsr();
+        }
     }
     s->tr_first_h[nsub] = (int)tr_sub.size();
     for (int f = 0; f < 2; ++f) s->cu_first_h[f][nsub] = (int)cpl[f].unit.size();
@@ -3614,6 +3586,123 @@ int s2l_gpu_setup_end(s2l_setup* s)
                 s->kc_max = kc;
     if (level) s->kc_max = s->lay[0].kc_max;  // (as many slots in layout 1)
     CUDA_OK(s, cudaStreamSynchronize(s->setup_stream));
+    s2l_work* w0 = nullptr;
+    RET_IF(work_create(s, &w0));
+    if (s->user_stream) w0->stream = s->user_stream;
+    s->works.push_back(w0);
+    s->busy.push_back(0);
+    return S2L_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int s2l_gpu_setup_end(s2l_setup* s)
+{
+    if (!s) return S2L_ERR_BADARG;
+    if (s->ended) return s->fail(S2L_ERR_STATE, "setup_end called twice");
+    if (!s->have_A) return s->fail(S2L_ERR_STATE, "set_matrix was not called");
+    if (cudaSetDevice(s->ctx->device) != cudaSuccess) return S2L_ERR_CUDA;
+    const int nsub = s->nsub;
+    if (s->local_kind == 1 && s->opt_refactor)
+        return s->fail(S2L_ERR_BADARG, "the option refactor needs exact local factors");
+    // ---- ownership checks: contiguous ranges covering [0, n)
+    {
+        int64_t next = 0;
+        for (int i = 0; i < nsub; ++i) {
+            if (!s->hs[i].set) return s->fail(S2L_ERR_STATE, "subdomain " + std::to_string(i) + " was not added");
+            if (s->hs[i].begin != next) return s->fail(S2L_ERR_BADARG, "owned ranges must be contiguous in subdomain order");
+            next += s->hs[i].n_owned;
+        }
+        if (next != s->n) return s->fail(S2L_ERR_BADARG, "owned ranges do not cover [0, n)");
+    }
+    if (s->coarse != S2L_COARSE_NONE) {
+        if (!s->have_coarse) return s->fail(S2L_ERR_STATE, "set_coarse was not called");
+        if (s->coff[0] != 0 || s->coff[nsub] != s->n0) return s->fail(S2L_ERR_BADARG, "coarse offsets inconsistent with n0");
+        for (int i = 0; i < nsub; ++i)
+            if (s->coff[i + 1] - s->coff[i] != s->hs[i].m)
+                return s->fail(S2L_ERR_BADARG, "coarse offsets do not match the basis sizes");
+    }
+    const bool boolean = s->pou == S2L_POU_BOOLEAN;
+    s->need_copies = !(boolean && s->one_level == S2L_ONE_LEVEL_RAS);
+
+    // ---- global matrix
+    {
+        std::vector<int32_t> rp(s->n + 1);
+        for (int64_t r = 0; r <= s->n; ++r) rp[r] = (int32_t)s->A.rp[r];
+        s->nnz = s->A.rp[s->n];
+        RET_IF(upload(s, &s->d_rp, rp));
+        RET_IF(upload(s, &s->d_ci, s->A.ci));
+        RET_IF(upload(s, &s->d_av, s->A.v));
+        std::vector<double> rowsum(s->n, 0.0);  // A 1, summed in row order as a CSR product does
+        for (int64_t r = 0; r < s->n; ++r)
+            for (int64_t e = s->A.rp[r]; e < s->A.rp[r + 1]; ++e) rowsum[r] += s->A.v[e];
+        RET_IF(upload(s, &s->d_rowsum, rowsum));
+        const double avg = (double)s->nnz / (double)s->n;
+        // lanes per row for about four entries per lane, between 2 and 32 (each lane with four
+        // entries in flight: on a 7-point matrix 2 lanes per row beat the chunk mode, a warp per 32
+        // rows with coalesced entry loads, spmv_tpr 1, by 1.3x for one column and 1.5x for four)
+        int tpr = 2;
+        while (tpr < 32 && tpr * 4 < avg) tpr *= 2;
+        s->tpr = s->opt_tpr ? s->opt_tpr : tpr;
+    }
+
+    // ---- full U of every subdomain
+    std::vector<HostCsr> Us(nsub);
+    // per subdomain and independent of the others: on several host threads
+    std::vector<char> ldlt_bad(nsub, 0);
+    parallel_for(nsub, [&](int i) {
+        HostSub& h = s->hs[i];
+        const int nl = h.n_local();
+        if (h.amg) return;
+        if (h.kind == S2L_FACTOR_LU) {
+            Us[i] = std::move(h.U);
+        } else {
+            Us[i] = transpose_lower(h.L, nl, nullptr);
+            if (h.kind == S2L_FACTOR_LDLT) {
+                bool missing = false;
+                for (int r = 0; r < nl; ++r) {
+                    bool f = false;
+                    for (int64_t e = Us[i].rp[r]; e < Us[i].rp[r + 1]; ++e) {
+                        if (Us[i].ci[e] == r) {
+                            Us[i].v[e] = h.d[r];
+                            f = true;
+                        } else {
+                            Us[i].v[e] *= h.d[r];
+                        }
+                    }
+                    missing = missing || !f;
+                }
+                if (missing) {
+                    ldlt_bad[i] = 1;
+                    return;
+                }
+            }
+        }
+    });
+    for (int i = 0; i < nsub; ++i)
+        if (ldlt_bad[i]) return s->fail(S2L_ERR_BADARG, "LDLT: L must store its unit diagonal");
+    // ---- layouts.  The fastest ones are not the smallest; where they do not fit the memory, the smallest are
+    // tried, from the same factors: those are kept on the host meanwhile, but only where a generous estimate
+    // of what could be allocated (three copies of every entry, the largest tails, the plan) does not fit.
+    const double rsz = s->real == S2L_REAL_F32 ? 4.0 : 8.0;
+    double most = 0.0;
+    for (int i = 0; i < nsub; ++i) {
+        const HostSub& h = s->hs[i];
+        const double e = (double)h.L.ci.size() + (double)Us[i].ci.size(), nl = h.n_local();
+        const double t = std::min(nl, (double)std::max({s->opt_tail_max, s->opt_tail_rows, s->opt_tail_min}));
+        most += e * (3.0 * (rsz + 4.0) + (s->opt_refactor ? 80.0 : 0.0)) + t * t * (2.0 * rsz + 24.0) +
+                nl * (16.0 * h.m + 400.0);
+    }
+    const bool keep = s->local_kind == 0 && most + (double)s->nnz * 16.0 + 32.0 * s->n0 * s->n0 > memory_left(s->ctx);
+    const size_t mark = s->allocs.size(), before = s->bytes;
+    int rc = setup_layouts(s, Us, false, keep);
+    if (rc == S2L_ERR_OOM && keep) {
+        drop_layouts(s, mark, before);
+        rc = setup_layouts(s, Us, true, false);
+    }
+    RET_IF(rc);
     // host staging no longer needed
     s->A.ci = {};  // the row pointers stay: s2l_gpu_update_matrix recomputes the row sums with them
     s->A.v = {};
@@ -3623,11 +3712,6 @@ int s2l_gpu_setup_end(s2l_setup* s)
         h.V.clear();
         h.V.shrink_to_fit();
     }
-    s2l_work* w0 = nullptr;
-    RET_IF(work_create(s, &w0));
-    if (s->user_stream) w0->stream = s->user_stream;
-    s->works.push_back(w0);
-    s->busy.push_back(0);
     s->ended = true;
     return S2L_OK;
 }
@@ -3653,12 +3737,7 @@ int s2l_gpu_setup_destroy(s2l_setup* s)
         s->ctx->used -= std::min(s->ctx->used, s->bytes);
     }
     if (s->setup_stream) cudaStreamDestroy(s->setup_stream);
-    for (int q = 0; q < s2l_setup::Refac::RF_STREAMS; ++q) {
-        if (s->rf.tsolver[q]) cusolverDnDestroy(s->rf.tsolver[q]);
-        if (s->rf.tstream[q]) cudaStreamDestroy(s->rf.tstream[q]);
-    }
-    for (auto e : s->rf.tev)
-        if (e) cudaEventDestroy(e);
+    refactor_release(s);
     delete s;
     return S2L_OK;
 }
