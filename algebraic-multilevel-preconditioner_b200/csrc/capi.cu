@@ -52,6 +52,7 @@ struct s2l_ctx {
     std::string err;
     std::mutex mu;
     std::vector<s2l_setup*> spares;  // setups that hold a second layout (s2l_setup::spare; under mu)
+    int spare_wanted = 0;            // allocations that wait for one of them (under mu)
     s2l_serve* serve = nullptr;
     // device address of the static scratch of s2l_gpu_coarse_apply_noalloc, looked up by the first
     // such call on this context (with its device current); a context created after a reset of the
@@ -452,8 +453,7 @@ bool give_back_spare(s2l_ctx* c)
 
 thread_local size_t t_refused = 0;  // size of this thread's last allocation over the budget (0: cudaMalloc failed)
 
-// After a refused allocation: whether second layouts that calls are using would make room for it.  They come
-// free when those calls end; an allocation waits for that, S2L_SPARE_WAIT_S seconds at most.
+// After a refused allocation: whether second layouts that calls are using would make room for it
 bool spare_would_do(s2l_ctx* c)
 {
     std::lock_guard<std::mutex> g(c->mu);
@@ -488,15 +488,41 @@ int ctx_alloc(s2l_ctx* c, void** p, size_t bytes)
     return S2L_ERR_OOM;
 }
 
+// A wait for second layouts in use: the last call of a setup gives its own back when it ends (Lease), as long as
+// somebody waits; S2L_SPARE_WAIT_S seconds at most
+struct SpareWait {
+    s2l_ctx* c;
+    const std::chrono::steady_clock::time_point end = std::chrono::steady_clock::now() + std::chrono::seconds(S2L_SPARE_WAIT_S);
+    bool counted = false;
+    explicit SpareWait(s2l_ctx* c_) : c(c_) {}
+    bool worth()  // after a refused allocation
+    {
+        if (!spare_would_do(c) || std::chrono::steady_clock::now() >= end) return false;
+        std::lock_guard<std::mutex> g(c->mu);
+        c->spare_wanted += counted ? 0 : 1;
+        return counted = true;
+    }
+    ~SpareWait()
+    {
+        std::lock_guard<std::mutex> g(c->mu);
+        c->spare_wanted -= counted ? 1 : 0;
+    }
+};
+
+// an allocation of the setup phase (no lock is held), with such a wait
+template <typename F>
+int setup_alloc(s2l_ctx* c, F&& alloc)
+{
+    SpareWait wait(c);
+    int rc;
+    while ((rc = alloc()) == S2L_ERR_OOM && wait.worth()) std::this_thread::sleep_for(std::chrono::milliseconds(1));
+    return rc;
+}
+
 int dev_alloc(s2l_setup* s, void** p, size_t bytes)
 {
     if (bytes == 0) bytes = 16;
-    const auto deadline = std::chrono::steady_clock::now() + std::chrono::seconds(S2L_SPARE_WAIT_S);
-    int rc;
-    while ((rc = ctx_alloc(s->ctx, p, bytes)) == S2L_ERR_OOM && spare_would_do(s->ctx) &&
-           std::chrono::steady_clock::now() < deadline)
-        std::this_thread::sleep_for(std::chrono::milliseconds(2));  // (no lock is held here)
-    RET_IF(rc);
+    RET_IF(setup_alloc(s->ctx, [&] { return ctx_alloc(s->ctx, p, bytes); }));
     s->allocs.push_back(*p);
     s->bytes += bytes;
     return S2L_OK;
@@ -2165,7 +2191,7 @@ struct Lease {
         }
         std::unique_lock<std::mutex> g(s->wmu);
         const auto deadline = std::chrono::steady_clock::now() + std::chrono::seconds(S2L_ADMIT_WAIT_S);
-        const auto spare_deadline = std::chrono::steady_clock::now() + std::chrono::seconds(S2L_SPARE_WAIT_S);
+        SpareWait spare(s->ctx);
         auto take = [&](size_t i) -> int {  // reserve workspace i and prepare it (lock released meanwhile)
             s->busy[i] = 1;
             s2l_work* cand = s->works[i];
@@ -2204,8 +2230,8 @@ struct Lease {
             }
             bool anybusy = false;
             for (char b : s->busy) anybusy = anybusy || b;
-            if (!anybusy && spare_would_do(s->ctx) && std::chrono::steady_clock::now() < spare_deadline) {
-                s->wcv.wait_for(g, std::chrono::milliseconds(2));
+            if (!anybusy && spare.worth()) {
+                s->wcv.wait_for(g, std::chrono::milliseconds(1));
                 continue;
             }
             if (!anybusy || s->wcv.wait_until(g, deadline) == std::cv_status::timeout) {
@@ -2228,10 +2254,12 @@ struct Lease {
     ~Lease()
     {
         if (idx < 0) return;
+        bool wanted;
         {
             std::lock_guard<std::mutex> a(s->ctx->mu);
-            --s->active;
+            wanted = --s->active == 0 && s->ctx->spare_wanted > 0;
         }
+        if (wanted) give_back_spare(s->ctx);
         {
             std::lock_guard<std::mutex> g(s->wmu);
             s->busy[idx] = 0;
@@ -3587,7 +3615,7 @@ int setup_layouts(s2l_setup* s, std::vector<HostCsr>& Us, bool smallest, bool ke
     if (level) s->kc_max = s->lay[0].kc_max;  // (as many slots in layout 1)
     CUDA_OK(s, cudaStreamSynchronize(s->setup_stream));
     s2l_work* w0 = nullptr;
-    RET_IF(work_create(s, &w0));
+    RET_IF(setup_alloc(s->ctx, [&] { return work_create(s, &w0); }));
     if (s->user_stream) w0->stream = s->user_stream;
     s->works.push_back(w0);
     s->busy.push_back(0);

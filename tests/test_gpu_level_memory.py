@@ -116,8 +116,10 @@ def test_another_setup_takes_its_place_and_refactorization_goes_on(case):
     ctx.close()
 
 
-def test_a_layout_in_use_is_waited_for(case):
-    """Requests run on the setup while another one is uploaded into the memory of its second layout."""
+@pytest.mark.parametrize("requests", [6, 100])
+def test_a_layout_in_use_is_waited_for(case, requests):
+    """Requests run on the setup, one right after the other, while another setup is uploaded into the memory of
+    its second layout."""
     from s2l_b200 import capi
     w, st, o, full, _ = case
     _, st2 = small_setup("bubbles3d")
@@ -133,7 +135,7 @@ def test_a_layout_in_use_is_waited_for(case):
     ctx = capi.Context(0, hbm_budget=full + solve + other - 4096)
     ctx.serve_start(1, batching=0)
     g = capi.GpuSetup(ctx, st)
-    tickets = [g.submit(st.b, restart=w.restart, rtol=1e-8) for _ in range(6)]
+    tickets = [g.submit(st.b, restart=w.restart, rtol=1e-8) for _ in range(requests)]
     g2 = capi.GpuSetup(ctx, st2)
     xs = []
     for t in tickets:
