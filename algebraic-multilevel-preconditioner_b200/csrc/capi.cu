@@ -4168,6 +4168,7 @@ int s2l_gpu_setup_stat(const s2l_setup* s, const char* name, double* value)
     else if (n == "sweep_group") *value = (double)s->sweep_group;
     else if (n == "smem_bytes") *value = (double)s->smem_bytes;
     else if (n == "level_sweeps") *value = (double)(s->nlay > 0 ? s->lay[0].cs : 0);
+    else if (n == "level_slots") *value = (double)(s->nlay > 0 ? s->lay[0].slots : 0);
     else if (n == "level_layouts") *value = (double)s->nlay.load();
     else if (n == "levels_max") *value = (double)s->st_levels_max;
     else if (n == "chain_blocks") *value = (double)s->st_blocks;

@@ -254,7 +254,7 @@ int s2l_gpu_refactor(s2l_setup* s, const double* val, int ptr_kind);
 int s2l_gpu_setup_bytes(const s2l_setup* s, size_t* bytes);
 /* Layout statistics after setup_end: "sparse_nnz", "coupling_nnz", "dense_entries", "tail_rows",
    "sweep_group", "smem_bytes", "level_sweeps" (CTAs per subdomain of the level sweeps; 0: dataflow
-   sweeps), "level_layouts" (2: blocks of columns have a layout of their own; it is given back, at any
+   sweeps), "level_slots" (values a column takes in the shared memory of their CTAs), "level_layouts" (2: blocks of columns have a layout of their own; it is given back, at any
    time no call runs on the setup, when an allocation of the context needs its memory, and blocks then
    run on layout 1, their sums in another order), "levels_max" / "levels_mean" (dependency levels of a sparse sweep,
    largest and mean over subdomains and both factors), "chain_blocks", "sweep_tasks" and
