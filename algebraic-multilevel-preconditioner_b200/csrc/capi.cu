@@ -1191,7 +1191,7 @@ int upload_real(s2l_setup* s, void** dst, const std::vector<double>& v)
     return S2L_OK;
 }
 
-// ------------------------------------------------------------------------------ profiling
+// ------------------------------------------------------------------------------ level layouts
 // widest lane group of a row of the level sweeps
 int level_group(const s2l_setup* s) { return s->opt_group ? s->opt_group : 32; }
 
@@ -1409,6 +1409,7 @@ int build_level_layouts(s2l_setup* s, const std::vector<HostCsr>& Us, const std:
     return S2L_OK;
 }
 
+// ------------------------------------------------------------------------------ calls, workspaces, profiling
 int check_ready(s2l_setup* s)
 {
     if (!s) return S2L_ERR_BADARG;
@@ -1778,12 +1779,19 @@ int ensure_block(s2l_work* w, int K, int m, bool flex)
     return S2L_OK;
 }
 
+// SMs of the context's device (a B200's where the device does not say)
+int device_sms(const s2l_setup* s)
+{
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->ctx->device) != cudaSuccess || sms <= 0) sms = 148;
+    return sms;
+}
+
 // Widest block that keeps one wave of sparse-sweep CTAs: K/KC CTAs per subdomain on the SMs.
 int block_width_best(s2l_setup* s)
 {
     if (s->opt_block_width > 0) return s->opt_block_width;
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->ctx->device) != cudaSuccess || sms <= 0) sms = 148;
+    const int sms = device_sms(s);
     const int kc = s->need_gflags ? 1 : s->kc_max;
     int w = kc * std::max(1, sms / std::max(s->nsub, 1));
     int p = 1;
@@ -2167,9 +2175,6 @@ void work_destroy(s2l_work* w)
     delete w;
 }
 
-// A free workspace for one solve-phase call: workspace 0 when it is free (it carries the caller's
-// stream and timers), another free one, or a new one when every workspace is busy (concurrent
-// calls on one setup from several threads).
 // A workspace for one solve-phase call: workspace 0 when it is free (it carries the caller's
 // stream and timers), another free one, or a new one when every workspace is busy (concurrent
 // calls on one setup from several threads).  `prepare` allocates what the call needs on the
@@ -2887,7 +2892,7 @@ int setup_layouts(s2l_setup* s, std::vector<HostCsr>& Us, bool smallest, bool ke
         // steps) 75, 79, 85, -, in FP64 (0.9 steps) 105, 104, 109, -; 32^3 / 8 (1.2 steps) 119, 112, 121, -;
         // 40^3 / 32 (2 steps) 133, 131, 130, -; 48^3 / 8 (10 steps) -, 280, 275, 293; 100^3 / 64 (109 steps) -,
         // 1026, 1003, 997.
-        const double steps = (double)cnt / (128.0 * 32.0 * S2L_SMS);
+        const double steps = (double)cnt / (128.0 * 32.0 * device_sms(s));
         for (auto& c : cpl) {
             c.real_bytes = rs;
             c.per_lane = steps >= 32.0 ? 32 : smallest || steps >= 4.0 ? 16 : steps >= 0.75 ? 4 : 2;
@@ -3437,9 +3442,7 @@ int setup_layouts(s2l_setup* s, std::vector<HostCsr>& Us, bool smallest, bool ke
         RET_IF(dev_alloc(s, reinterpret_cast<void**>(&R.err), sizeof(int)));
         {
             // clusters of 4 or 2 CTAs per subdomain when they fit the SMs at once, else one
-            int sms = 0;
-            if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->ctx->device) != cudaSuccess || sms <= 0)
-                sms = 148;
+            const int sms = device_sms(s);
             R.cs = nsub * 4 <= sms ? 4 : (nsub * 2 <= sms ? 2 : 1);
             int smax = 1;
             for (int sz : R.sz) smax = std::max(smax, sz);

@@ -2,7 +2,9 @@
 //
 // All reductions are deterministic: every reduction-producing kernel runs on a fixed grid of
 // S2L_NB_RED blocks, writes one partial per block and column, and reduce_kernel sums them in a
-// fixed order.  The same input therefore gives bitwise-identical results, alone or in a batch.
+// fixed order.  The same call on the same setup therefore gives the same bits every time, whatever else
+// runs.  Blocks of another width may sum in another order (the couplings, the dense tails and the
+// layouts of the level sweeps go by the number of columns).
 #include "s2l_internal.cuh"
 
 #include <type_traits>

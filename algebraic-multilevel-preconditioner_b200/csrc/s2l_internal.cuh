@@ -36,7 +36,6 @@
 #define S2L_SPIN_SLEEP_NS 0   // pause of a sweep warp after a poll that found a column not ready (ns; 0 = none)
 #endif
 #define S2L_SPIN_LIMIT (1 << 24)  // polls of one ready flag before a sweep gives up (error 1)
-#define S2L_SMS 148           // SMs that rules on sizes count on
 #define S2L_BS_LEVEL 512      // threads of a CTA of the level sweeps (level_sweep.cu)
 #define S2L_LEVEL_HOP_US 2.0  // the tail split's time of a level of a level sweep (hop_us default)
 #define S2L_LEVEL_CAP 64      // rows of a block of the level sweeps, at most
