@@ -2854,9 +2854,10 @@ int setup_layouts(s2l_setup* s, std::vector<HostCsr>& Us, bool smallest, bool ke
     split(false, 0);
     // Few levels stay with the flags: a hand-over costs both about the same (1 us), but a level sweep's
     // stages come twice a level, and the longer tail that its split takes costs what the shorter chain
-    // saves.  Local solves in us, dataflow and level sweeps: 16 levels (bubbles3d 24^3 / 8) 68 and 76,
-    // 23 (40^3 / 32) 138 and 158, 24 (32^3 / 8) 124 and 139, 32 (36^3 / 8) 199 and 170, 40 (40^3 / 8)
-    // 275 and 205, 63 (convdiff3d 32^3 / 12) 262 and 157, 77 (poisson2d 200^2 / 8) 224 and 117.
+    // saves.  Local solves of one column in us, dataflow and level sweeps: 16 levels (bubbles3d 24^3 / 8) 65
+    // and 72, 23 (40^3 / 32) 132 and 149, 24 (32^3 / 8) 112 and 134, 32 (36^3 / 8) 192 and 162, 40 (40^3 / 8)
+    // 266 and 194, 63 (convdiff3d 32^3 / 12) 249 and 150, 77 (poisson2d 200^2 / 8) 220 and 117.  (Four columns
+    // gain everywhere, 108 and 69, 204 and 174, 234 and 125 on the first three, at two to three times the memory.)
     if (level) {
         const std::vector<int> dataflow = Ts;
         const int flags = deepest;

@@ -13,10 +13,10 @@
 // waited some 1000 cycles for its loads: a warp has six scoreboards for all of them.)
 //
 // Measured on one B200: local solve of all subdomains in us, CUDA events, dataflow sweeps (kernels.cu)
-// and level sweeps, one column and four columns:
-//   bubbles3d 48^3 / 8     FP64   498 -> 285    617 -> 420      poisson2d 200^2 / 8  FP64  224 -> 117   492 -> 147
-//   bubbles3d 48^3 / 8     FP32   353 -> 225    788 -> 340      convdiff3d 48^3 / 12 FP32 1043 -> 330  1875 -> 562
-//   bubbles3d 100^3 / 64   FP64  1319 -> 1079  2690 -> 2440     bubbles3d 100^3 / 64 FP32  917 -> 813  1527 -> 1324
+// and level sweeps, one column and four columns, couplings and tails the same in both:
+//   bubbles3d 48^3 / 8     FP64   481 -> 271    502 -> 328      poisson2d 200^2 / 8  FP64  220 -> 117    495 -> 144
+//   bubbles3d 48^3 / 8     FP32   341 -> 215    720 -> 269      convdiff3d 48^3 / 12 FP32 1014 -> 309   1770 -> 481
+//   bubbles3d 100^3 / 64   FP64  1210 -> 983   1900 -> 1790     bubbles3d 100^3 / 64 FP32  787 -> 684   1025 -> 895
 // (the whole local solve; on 100^3 / 64 FP32 the two sweeps take 145 and 174 us of it).
 #include "s2l_internal.cuh"
 

@@ -91,3 +91,19 @@ def test_concurrent_callers(case):
             got = list(pool.map(lambda b: (g.apply(b), g.gmres(b, **kw)[0], g.apply_block(B[:4])), B))
             for a, q in zip(alone, got):
                 assert all(np.array_equal(u, v) for u, v in zip(a, q))
+
+
+def test_time_loop():
+    """A sequence with refactorizations: levels and iterations (one more or less) of the dataflow sweeps."""
+    from s2l_b200 import capi
+    from s2l_b200 import workloads as W
+    from s2l_b200.time_loop import TimeLoopConfig, levels, run_time_loop
+    w = W.bubbles3d(12, 8, nbubbles=6, overlap=1)
+    w.opts.nev = 8
+    ctx = capi.Context(0)
+    cfg = TimeLoopConfig(steps=3, correctors=2, reuse="refactor")
+    on, off = (run_time_loop(w, cfg, ctx=ctx, workers=1, options={"level_sweeps": v}) for v in (1, 0))
+    assert levels(on) == levels(off) == "201010"
+    for a, b in zip(on, off):
+        assert a.converged and a.true_rel_residual <= 1.1 * w.rtol and abs(a.iterations - b.iterations) <= 1
+    ctx.close()
