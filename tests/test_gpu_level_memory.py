@@ -149,3 +149,22 @@ def test_a_layout_in_use_is_waited_for(case, requests):
     check(g, st, o, widths=(1, 2))
     g.close()
     ctx.close()
+
+
+def test_budgets_between_one_layout_and_two(case):
+    """The second layout's own allocations fail at any of their steps; down to the setup with one layout."""
+    from s2l_b200 import capi
+    _, st, o, full, _ = case
+    ctx = capi.Context(0, hbm_budget=full - 4096)
+    g = capi.GpuSetup(ctx, st)
+    one = g.device_bytes()
+    assert g.stat("level_layouts") == 1
+    g.close()
+    ctx.close()
+    for part in (0.9, 0.7, 0.5, 0.3, 0.1, 0.0):
+        ctx = capi.Context(0, hbm_budget=one + int(part * (full - one)))
+        g = capi.GpuSetup(ctx, st)
+        assert g.stat("level_layouts") == 1 and g.device_bytes() == one
+        check(g, st, o, widths=(1,))
+        g.close()
+        ctx.close()
