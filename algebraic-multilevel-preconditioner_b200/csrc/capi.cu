@@ -53,6 +53,8 @@ struct s2l_ctx {
     std::mutex mu;
     std::vector<s2l_setup*> spares;  // setups that hold a second layout (s2l_setup::spare; under mu)
     int spare_wanted = 0;            // allocations that wait for one of them (under mu)
+    size_t spare_freeing = 0;        // bytes of second layouts being freed
+    unsigned long spares_given = 0;  // second layouts given back so far (under mu)
     s2l_serve* serve = nullptr;
     // device address of the static scratch of s2l_gpu_coarse_apply_noalloc, looked up by the first
     // such call on this context (with its device current); a context created after a reset of the
@@ -257,6 +259,8 @@ struct s2l_setup {
     std::condition_variable wcv;  // a workspace came free
     std::vector<s2l_work*> works;
     std::vector<char> busy;
+    bool admitting = false;      // a call is looking for its workspace
+    unsigned long released = 0;  // leases that ended
     cudaStream_t user_stream = nullptr;  // s2l_gpu_set_stream: used by workspace 0
     unsigned prof_mask = 0;              // s2l_gpu_profile_enable: inherited by new workspaces
 
@@ -441,6 +445,7 @@ bool give_back_spare(s2l_ctx* c)
         gone.swap(s->spare);
         bytes = s->spare_bytes;
         s->spare_bytes = 0;
+        c->spare_freeing += bytes;
         s->nlay = 1;
         s->lay[1] = {};
     }
@@ -448,19 +453,12 @@ bool give_back_spare(s2l_ctx* c)
     for (void* p : gone) cudaFree(p);
     std::lock_guard<std::mutex> g(c->mu);
     c->used -= std::min(c->used, bytes);
+    c->spare_freeing -= bytes;
+    ++c->spares_given;
     return true;
 }
 
 thread_local size_t t_refused = 0;  // size of this thread's last allocation over the budget (0: cudaMalloc failed)
-
-// After a refused allocation: whether second layouts that calls are using would make room for it
-bool spare_would_do(s2l_ctx* c)
-{
-    std::lock_guard<std::mutex> g(c->mu);
-    size_t sum = 0;
-    for (const s2l_setup* s : c->spares) sum += s->spare_bytes;
-    return sum > 0 && t_refused > 0 && c->used - std::min(c->used, sum) + t_refused <= c->budget;
-}
 
 // device memory within the context's budget; second layouts that idle setups hold make room for it
 int ctx_alloc(s2l_ctx* c, void** p, size_t bytes)
@@ -494,11 +492,25 @@ struct SpareWait {
     s2l_ctx* c;
     const std::chrono::steady_clock::time_point end = std::chrono::steady_clock::now() + std::chrono::seconds(S2L_SPARE_WAIT_S);
     bool counted = false;
-    explicit SpareWait(s2l_ctx* c_) : c(c_) {}
-    bool worth()  // after a refused allocation
+    unsigned long seen = 0;
+    explicit SpareWait(s2l_ctx* c_) : c(c_)
     {
-        if (!spare_would_do(c) || std::chrono::steady_clock::now() >= end) return false;
         std::lock_guard<std::mutex> g(c->mu);
+        seen = c->spares_given;
+    }
+    // After a refused allocation: whether to try it again, because a layout was given back since the last
+    // attempt began or because those in use would make room for it
+    bool worth()
+    {
+        std::lock_guard<std::mutex> g(c->mu);
+        if (c->spares_given != seen) {
+            seen = c->spares_given;
+            return true;
+        }
+        size_t sum = c->spare_freeing;
+        for (const s2l_setup* s : c->spares) sum += s->spare_bytes;
+        if (sum == 0 || t_refused == 0 || c->used - std::min(c->used, sum) + t_refused > c->budget) return false;
+        if (std::chrono::steady_clock::now() >= end) return false;
         c->spare_wanted += counted ? 0 : 1;
         return counted = true;
     }
@@ -2183,6 +2195,8 @@ void work_destroy(s2l_work* w)
 // Admission by HBM footprint: when those allocations do not fit the context's budget, the call
 // waits for a busy workspace of this setup to come free (it usually has them already) and tries
 // again; it fails with S2L_ERR_OOM only when no workspace is busy or after S2L_ADMIT_WAIT_S seconds.
+// One call of a setup at a time allocates: two that try at once would stand in each other's way with what
+// each has allocated so far, and both be refused.
 struct Lease {
     s2l_setup* s;
     s2l_work* w = nullptr;
@@ -2206,44 +2220,54 @@ struct Lease {
             if (r != S2L_OK) s->busy[i] = 0;
             return r;
         };
+        auto free_to_admit = [&] { return !s->admitting; };
+        if (!s->wcv.wait_until(g, deadline, free_to_admit)) {
+            rc = s->fail(S2L_ERR_OOM, "waited too long for another call's allocations");
+            return;
+        }
+        s->admitting = true;
         for (;;) {
-            for (size_t i = 0; i < s->works.size() && idx < 0; ++i) {
+            const unsigned long seen = s->released;
+            int r = S2L_OK;
+            bool idle = false;
+            for (size_t i = 0; i < s->works.size() && idx < 0 && (r == S2L_OK || r == S2L_ERR_OOM); ++i) {
                 if (s->busy[i]) continue;
-                const int r = take(i);
+                idle = true;
+                r = take(i);
                 if (r == S2L_OK) idx = (int)i;
-                else if (r != S2L_ERR_OOM) {
-                    rc = r;
-                    return;
+            }
+            if (!idle) {  // (beside an idle workspace a new one would need more memory yet)
+                s2l_work* nw = nullptr;
+                r = work_create(s, &nw);
+                if (r == S2L_OK) {
+                    s->works.push_back(nw);
+                    s->busy.push_back(0);
+                    const size_t i = s->works.size() - 1;
+                    r = take(i);
+                    if (r == S2L_OK) idx = (int)i;
                 }
             }
             if (idx >= 0) break;
-            s2l_work* nw = nullptr;
-            int r = work_create(s, &nw);
-            if (r == S2L_OK) {
-                s->works.push_back(nw);
-                s->busy.push_back(0);
-                const size_t i = s->works.size() - 1;
-                r = take(i);
-                if (r == S2L_OK) {
-                    idx = (int)i;
-                    break;
-                }
+            if (r == S2L_ERR_OOM && s->released != seen) continue;  // a workspace came free meanwhile
+            bool leased = false;
+            for (char b : s->busy) leased = leased || b;
+            if (r != S2L_ERR_OOM || (!leased && !spare.worth())) {
+                rc = r;  // the message of the failed allocation stays in last_error
+                break;
             }
-            if (r != S2L_ERR_OOM) {
-                rc = r;
+            // the end of a call, of this setup or (a moment) of one whose second layout is wanted; others try meanwhile
+            s->admitting = false;
+            s->wcv.notify_all();
+            if (!leased) s->wcv.wait_for(g, std::chrono::milliseconds(1));
+            if (!s->wcv.wait_until(g, deadline, [&] { return !s->admitting && (!leased || s->released != seen); })) {
+                rc = S2L_ERR_OOM;
                 return;
             }
-            bool anybusy = false;
-            for (char b : s->busy) anybusy = anybusy || b;
-            if (!anybusy && spare.worth()) {
-                s->wcv.wait_for(g, std::chrono::milliseconds(1));
-                continue;
-            }
-            if (!anybusy || s->wcv.wait_until(g, deadline) == std::cv_status::timeout) {
-                rc = S2L_ERR_OOM;  // the message of the failed allocation stays in last_error
-                return;
-            }
+            s->admitting = true;
         }
+        s->admitting = false;
+        s->wcv.notify_all();
+        if (idx < 0) return;
         w = s->works[idx];
         {
             std::lock_guard<std::mutex> a(s->ctx->mu);
@@ -2268,6 +2292,7 @@ struct Lease {
         {
             std::lock_guard<std::mutex> g(s->wmu);
             s->busy[idx] = 0;
+            ++s->released;
         }
         s->wcv.notify_all();
     }

@@ -168,3 +168,39 @@ def test_budgets_between_one_layout_and_two(case):
         check(g, st, o, widths=(1,))
         g.close()
         ctx.close()
+
+
+def test_a_waiting_call_takes_no_further_workspaces(case):
+    """A call whose Krylov basis misses the budget by a little waits for the second layout in use of another
+    setup; while it waits it must not pile up workspaces (each fits, none helps)."""
+    from s2l_b200 import capi
+    w, st, _, full, _ = case
+    w2, st2 = small_setup("bubbles3d")
+    kw2 = {"restart": 50, "rtol": 1e-8}
+    probe = capi.Context(0)
+    g = capi.GpuSetup(probe, st)
+    g.gmres(st.b, restart=w.restart, rtol=1e-8)
+    solve = g.device_bytes() - full
+    g2 = capi.GpuSetup(probe, st2)
+    upload = g2.device_bytes()
+    x0, _ = g2.gmres(st2.b, **kw2)
+    alone = g2.device_bytes()
+    g2.close()
+    g.close()
+    probe.close()
+    ctx = capi.Context(0, hbm_budget=full + solve + alone - 4096)
+    ctx.serve_start(1, batching=0)
+    g = capi.GpuSetup(ctx, st)
+    g2 = capi.GpuSetup(ctx, st2)
+    assert g.stat("level_layouts") == 2
+    tickets = [g.submit(st.b, restart=w.restart, rtol=1e-8) for _ in range(60)]
+    x, _ = g2.gmres(st2.b, **kw2)
+    assert np.array_equal(x, x0)
+    assert g.stat("level_layouts") == 1
+    assert g2.device_bytes() <= alone + (alone - upload)
+    for t in tickets:
+        assert t.wait(120.0)[2] == 0
+        t.free()
+    g2.close()
+    g.close()
+    ctx.close()
